@@ -15,6 +15,26 @@ k_apply(const ApplyArgs<R> a)
   apply_strip<R, NW>(a, blockIdx.x * NW, smem_raw);
 }
 
+// Double precision on the tensor cores (oz_apply.cuh): one CTA per SM, 16-column strips.
+__global__ void __launch_bounds__(TQR_THREADS, 1)
+k_apply_oz(const ApplyArgs<double> a)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  apply_strip<double, oz::kCols, true>(a, blockIdx.x * oz::kCols, smem_raw);
+}
+
+static cudaError_t launch_oz(ApplyArgs<double> a, cudaStream_t st) {
+  cudaError_t e = cudaFuncSetAttribute(k_apply_oz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::kSmem);
+  if (e != cudaSuccess) return e;
+  a.nw = oz::kCols;
+  a.stage_c = a.stage_v = a.stage_t = 1;   // of the DFMA path a strip may fall back to
+  k_apply_oz<<<(a.ncols + oz::kCols - 1) / oz::kCols, TQR_THREADS, oz::kSmem, st>>>(a);
+  count_launch();
+  return cudaGetLastError();
+}
+static_assert(sizeof(double) * ((size_t)257 * (oz::kIbMax + oz::kCols) + 3 * 32 * 32) <= oz::kSmem,
+              "the DFMA path's staged strip fits the same shared memory");
+
 // Fewest CTAs a stand-alone apply should run on before narrower strips are used.
 constexpr int kMinStripCtas = 32;
 
@@ -88,6 +108,9 @@ cudaError_t launch_apply(int mode, char side, char trans, int m, int n, int k, i
   ApplyArgs<R> a = make_apply_args<R>(mode, side, trans, m, n, k, ib, C, ldc, A1, lda1, V, ldv, T,
                                       ldt, &sm);
   a.tt = (mode == 1) ? tt : -1;
+  if constexpr (std::is_same<R, double>::value) {
+    if (oz::covers(a.mode, a.L, a.k, a.ib)) return launch_oz(a, st);
+  }
   if (sm > (size_t)TQR_SMEM_MAX) return cudaErrorInvalidValue;
   switch (a.nw) {
     case 16: return launch_nw<R, 16>(a, sm, st);

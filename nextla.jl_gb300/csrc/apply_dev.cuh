@@ -58,6 +58,12 @@ struct ApplyArgs {
                  // never read and region rows past tt + q are not touched
 };
 
+}  // namespace tqr
+
+#include "oz_apply.cuh"
+
+namespace tqr {
+
 // Phase 2 keeps op(T) W in registers (up to kW2Regs entries per thread) and
 // only needs a second W buffer beyond that.
 constexpr int kW2Regs = 4;
@@ -134,15 +140,20 @@ __device__ __forceinline__ void phase1_blocked_f32(const float *Vp, int ldvp, co
     for (int w = 0; w < 4; ++w) pg[(p0 + u) + 32 * (c0 + w)] = acc[u][w];
 }
 
-// Apply to the strip of columns [c0, c0 + NW) (clamped to ncols).  VEC:
-// 16-byte staging of C and V for FP32 elements (kernels with registers to
-// spare: the tensor-core tile kernel runs one CTA per SM).
+// Apply to the strip of columns [c0, c0 + NW) (clamped to ncols).  VEC: the
+// kernel runs one CTA per SM, with registers to spare.  FP32 elements then
+// take 16-byte staging of C and V; FP64 ones run on the tensor cores
+// (oz_apply.cuh, the kernel has oz::kSmem bytes of dynamic shared memory)
+// wherever the shape is covered.
 template <typename R, int NW, bool VEC = false>
 __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_raw)
 {
   const int tid = threadIdx.x;
   const int nwl = min(NW, a.ncols - c0);
   if (nwl <= 0) return;
+  if constexpr (VEC && std::is_same<R, double>::value && NW <= oz::kCols) {
+    if (oz::covers(a.mode, a.L, a.k, a.ib) && oz::strip<0>(a, c0, nwl, smem_raw)) return;
+  }
   const int L = a.L, ib = a.ib;
   const int ldw = ib;
   const int ldcs = odd_ld(L), ldvs = odd_ld(L);

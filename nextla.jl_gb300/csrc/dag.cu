@@ -796,6 +796,17 @@ static int launch_dag(const DagArgs<R> &a, size_t sm, double flops, cudaStream_t
   return e == cudaSuccess ? 0 : (int)e;
 }
 
+// Double precision: whether the strip updates run on the tensor cores
+// (oz_apply.cuh), which takes one CTA per SM; panel-step strips of few rows
+// stay on the DFMA loops either way.
+static bool dag_oz(const DagGeom &g) { return oz::covers(1, g.nb, g.nb, g.ib); }
+
+static int launch_dag_oz(const DagArgs<double> &a, size_t sm, double flops, cudaStream_t st, bool timed = true) {
+  sm = std::max(sm, oz::kSmem);
+  return a.g.nw == 16 ? launch_dag<double, 16, true>(a, sm, flops, st, timed)
+                      : launch_dag<double, 8, true>(a, sm, flops, st, timed);
+}
+
 template <typename R>
 static int tile_geqrf_dag(int m, int n, int nb, int ib, R *A, int lda, R *T, int ldt, R *tau,
                           int ldtau, void *work, size_t lwork, cudaStream_t st, int nrhs = 0,
@@ -863,6 +874,9 @@ static int tile_geqrf_dag(int m, int n, int nb, int ib, R *A, int lda, R *T, int
   const double flops = 2.0 * mn * kn * kn - 2.0 * kn * kn * kn / 3.0;
   if constexpr (std::is_same<R, float>::value) {
     if (g.tc) return launch_dag<R, 16, true>(a, sm, flops, st);
+  }
+  if constexpr (std::is_same<R, double>::value) {
+    if (dag_oz(g)) return launch_dag_oz(a, sm, flops, st);
   }
   return g.nw == 16 ? launch_dag<R, 16>(a, sm, flops, st) : launch_dag<R, 8>(a, sm, flops, st);
 }
@@ -972,6 +986,7 @@ static int tile_geqrf_noalloc(int m, int n, int nb, int ib, double *A, int lda, 
   a.timeout_ns = 20ull * 1000ull * 1000ull * 1000ull;
   const size_t sm = std::max({apply_smem_elems(nb, ib, g.nw, true, true, true) * sizeof(double),
                               panel_smem<double>(nb, ib, true, true), tsqrt_smem<double>(nb, ib, true)});
+  if (dag_oz(g)) return launch_dag_oz(a, sm, 0.0, st, false);
   return g.nw == 16 ? launch_dag<double, 16>(a, sm, 0.0, st, false)
                     : launch_dag<double, 8>(a, sm, 0.0, st, false);
 }

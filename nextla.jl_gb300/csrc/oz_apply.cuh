@@ -1,0 +1,560 @@
+// oz_apply.cuh -- FP64 block-reflector apply on the tensor cores, exactly.
+//
+// GB300 executes two FP64 FMAs per clock and SM, on either FP64 pipe, but
+// 1024 FP16 multiply-adds through mma.sync with FP32 accumulators.  The
+// trailing update of apply_strip (W = A1 + V^T C, W = op(T) W, A1 -= W,
+// C -= V W) is three products, so every operand is cut into seven 9-bit
+// integer digits (error-free transformation in the manner of K. Ozaki,
+// T. Ogita, S. Oishi, S. M. Rump, "Error-free transformations of matrix
+// multiplication by using fast routines of matrix multiplication and its
+// applications", Numer. Algorithms 59, 2012) and each product becomes 28 FP16
+// products of digit planes, i + j <= 6.  A digit is in [-256, 255], so 32
+// terms of up to 7 plane pairs sum to at most 7 * 2^21 < 2^24: every FP32
+// accumulation is exact, whatever its order.
+//
+// Number format.  Column c of [A1; C] is held as 64-bit fixed point with its
+// own power-of-two scale 2^s: s is the largest with ||column|| 2^s <= 2^60.98.
+// An orthogonal update keeps that norm, |W| <= 2 ||column||, so nothing leaves
+// the 62-bit range the digits cover; V (|v| < 1.94) is scaled by 2^61 and T
+// (|t| < 4) by 2^59.  A strip that is not such an update (an infinity or NaN,
+// exponents near the ends of the range, a V or T beyond those bounds, a sum
+// that overflows) is detected before anything is written and the caller runs
+// the DFMA path on it.  An element whose fixed-point value the update did not
+// change is not written, so rows that no reflector touches keep their bits.
+//
+// Accuracy.  With c the column's root mean square over r rows, the unit of
+// the fixed point is 2^-61 sqrt(r) c; the dropped digit products (i + j > 6)
+// add about 2^3.7 units to W and 2^2.2 to C, where the FP64 sums they replace
+// round 256 and 32 times at 2^-53: measured against 64-bit references the
+// results are as close or closer.
+//
+// Layout.  Warp w owns rows [32 w, 32 w + 32) of the strip in registers, as
+// the accumulator fragment of (V W)^T: lane (g, t) = (lane / 4, lane % 4)
+// holds columns g, g + 8 and rows 8 q + 2 t, 8 q + 2 t + 1, q = 0..3.  That
+// is also the B fragment of V^T C, so C's digits go from registers to the
+// tensor core without shared memory.  V's digits are warp-private too (the
+// same 32 rows), one plane of 32 reflectors x 32 rows per digit in 64-byte
+// rows whose 16-byte chunks are permuted by (row / 2) % 4: ldmatrix and
+// ldmatrix.trans then serve both products conflict-free.  Only W crosses
+// warps: 64-bit partial sums, then op(T) W on warps 0..3 (8 reflectors each),
+// whose digits every warp reads as the A fragment of (V W)^T.
+//
+// What bounds it, per 32-reflector block of a 256-row, 16-column strip: 3584
+// mma.sync (2 clk each on an SM) = 7.2 k clk, against 131 k clk of DFMAs.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+
+namespace tqr {
+
+template <typename R> struct ApplyArgs;
+
+namespace oz {
+
+constexpr int kCols = 16;              // strip columns
+constexpr int kRowsMax = 256;          // region rows: 32 per warp
+constexpr int kIbMax = 32;
+constexpr int kKMax = 256;             // reflectors of a mode 1 apply (A1 rows kept in shared memory)
+constexpr int kD = 7;                  // digits
+constexpr uint32_t kPlaneV = 32 * 64;  // one digit plane of a warp's V: 32 reflectors x 32 rows
+constexpr uint32_t kWarpV = kD * kPlaneV;
+constexpr uint32_t kPlaneW = 16 * 64;
+constexpr int kLdWp = 36, kLdW1 = 40;
+// shared memory: V digits | T digits | W digits | partial W | W | A1 | reductions
+constexpr size_t kOffT = 8 * (size_t)kWarpV;
+constexpr size_t kOffW = kOffT + kD * (size_t)kPlaneV;
+constexpr size_t kOffWp = kOffW + kD * (size_t)kPlaneW;
+constexpr size_t kOffW1 = kOffWp + sizeof(long long) * 8 * kCols * kLdWp;
+constexpr size_t kOffA1 = kOffW1 + sizeof(long long) * kCols * kLdW1;
+constexpr size_t kOffRed = kOffA1 + sizeof(long long) * kCols * kKMax;
+constexpr size_t kSmem = kOffRed + sizeof(uint32_t) * kCols * 9;
+static_assert(kSmem <= TQR_SMEM_MAX, "one CTA's shared memory");
+
+// 256 in every digit: x + kBias has the digits of x plus 256, without carries
+constexpr unsigned long long kBias = 0x4020100804020100ull;
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: an integer |i| <= 2^22 is in the low bits of kMagic + i
+
+__device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                    uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+// x 2^s as an integer, rounded to nearest (RND) or towards zero; the caller
+// has checked that |x| 2^s < 2^62.
+template <bool RND>
+__device__ __forceinline__ long long to_fixed(double x, int s) {
+  const uint32_t hi = __double2hiint(x), lo = __double2loint(x);
+  const int e = (int)((hi >> 20) & 0x7ff);
+  unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
+  unsigned int t = (unsigned int)(1085 - s - e);      // m 2^-t is |x| 2^s; zeros and subnormals shift out
+  if (RND) {
+    // shr clamps the shift count, so a long shift gives zero
+    asm("shr.u64 %0, %1, %2;" : "=l"(m) : "l"(m), "r"(t - 1));
+    m = (m + 1) >> 1;
+  } else {
+    asm("shr.u64 %0, %1, %2;" : "=l"(m) : "l"(m), "r"(t));
+  }
+  const long long sg = (long long)((int)hi >> 31);
+  return ((long long)m ^ sg) - sg;
+}
+
+// Digit J (0 = lowest) of two biased fixed-point values as an f16 pair.
+template <int J>
+__device__ __forceinline__ uint32_t digit(unsigned long long a, unsigned long long b) {
+  const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+  uint32_t w;
+  // bytes J, J + 1 of each value hold the digit at bit J
+  if (J == 0) w = __byte_perm(al, bl, 0x5410);
+  if (J == 1) w = __byte_perm(al, bl, 0x6521) >> 1;
+  if (J == 2) w = __byte_perm(al, bl, 0x7632) >> 2;
+  if (J == 3) w = __byte_perm(__funnelshift_r(al, ah, 27), __funnelshift_r(bl, bh, 27), 0x5410);
+  if (J == 4) w = __byte_perm(ah, bh, 0x5410) >> 4;
+  if (J == 5) w = __byte_perm(ah, bh, 0x6521) >> 5;
+  if (J == 6) w = __byte_perm(ah, bh, 0x7632) >> 6;
+  w = (w & 0x01ff01ffu) | 0x64006400u;                // 1024 + digit + 256 in f16
+  uint32_t r;
+  asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0x65006500u));   // - 1280
+  return r;
+}
+
+// The seven digits of a pair, highest first, through put(plane, word).
+template <typename F>
+__device__ __forceinline__ void digits(unsigned long long a, unsigned long long b, F &&put) {
+  put(0, digit<6>(a, b));
+  put(1, digit<5>(a, b));
+  put(2, digit<4>(a, b));
+  put(3, digit<3>(a, b));
+  put(4, digit<2>(a, b));
+  put(5, digit<1>(a, b));
+  put(6, digit<0>(a, b));
+}
+
+template <typename F>
+__device__ __forceinline__ void init_acc(F (&acc)[kD][4]) {
+#pragma unroll
+  for (int d = 0; d < kD; ++d)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[d][e] = d < 2 ? kMagic : 0.0f;
+}
+
+// sum_d acc[d] 2^(SH - 9 d), rounded once below the unit; sets bad when the
+// value leaves (-2^62, 2^62).  Diagonals 0 and 1 (|sum| <= 2^22) were
+// accumulated on top of kMagic, so their integers are read from the bits.
+template <int SH>
+__device__ __forceinline__ long long recon(const float (&acc)[kD][4], int e, int &bad) {
+  const int i0 = __float_as_int(acc[0][e]) - 0x4B400000, i1 = __float_as_int(acc[1][e]) - 0x4B400000;
+  const int i2 = __float2int_rn(acc[2][e]), i3 = __float2int_rn(acc[3][e]), i4 = __float2int_rn(acc[4][e]);
+  const int i5 = __float2int_rn(fmaf(acc[5][e], (float)(1 << (SH - 45)), acc[6][e] * (1.0f / (float)(1 << (54 - SH)))));
+  long long r = (long long)i5;
+  r += (long long)i4 * (1ll << (SH - 36));
+  r += (long long)i3 * (1ll << (SH - 27));
+  r += (long long)i2 * (1ll << (SH - 18));
+  r += (long long)((i0 << (SH - 32)) + (i1 << (SH - 41))) << 32;
+  // |value| / 2^SH is within 26 / 512 of |i0 + i1 / 512|
+  const int top = i0 + (i1 >> 9);
+  constexpr int lim = (int)((1ll << (62 - SH)) * 0.99);
+  bad |= (top > lim) | (top < -lim);
+  return r;
+}
+
+// Byte offset of 16-bit element (row, k), k even, in a plane of 64-byte rows.
+__device__ __forceinline__ uint32_t plane_off(int row, int k) {
+  return (uint32_t)row * 64u + (uint32_t)((((k >> 3) ^ (row >> 1)) & 3) << 4) + (uint32_t)((k & 7) * 2);
+}
+
+// Whether the arguments are ones strip() covers; a property of the call, not
+// of the strip, so every driver of the same update takes the same path.
+// Below 48 rows or 12 reflectors the DFMA loops are the faster ones (the
+// fixed cost of a block is a few thousand clocks; see the figures in
+// apply_strip).
+__host__ __device__ inline bool covers(int mode, int L, int k, int ib) {
+  return ib <= kIbMax && L <= kRowsMax && (mode == 0 || k <= kKMax) && (ib < k ? ib : k) >= 8 && L >= 32;
+}
+
+// Applies to the strip of columns [c0, c0 + nwl).  False: the strip needs the
+// DFMA path; nothing has been written.  All threads get the same answer.
+template <int kUnused>
+__device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int L = a.L, ib = a.ib, k = a.k;
+  unsigned char *Vd = smem + (size_t)warp * kWarpV;
+  unsigned char *Td = smem + kOffT, *Wd = smem + kOffW;
+  long long *Wp = reinterpret_cast<long long *>(smem + kOffWp);
+  long long *W1 = reinterpret_cast<long long *>(smem + kOffW1);
+  long long *A1s = reinterpret_cast<long long *>(smem + kOffA1);
+  uint32_t *red = reinterpret_cast<uint32_t *>(smem + kOffRed);   // [warp 0..7, A1][column]
+  const bool tt = a.mode == 1 && a.tt >= 0;
+  const int Lt = tt ? min(L, a.tt + k) : L;            // rows any reflector touches
+  int bad = 0;
+
+  // ---- the strip, and A1's rows, from global memory ----
+  double *const Cg = a.C + (size_t)c0 * a.c_cs;
+  const bool vec = a.c_rs == 1 && ((uintptr_t)Cg & 15) == 0 && (a.c_cs & 1) == 0;
+  double x[2][4][2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t;
+      const double *p = Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs;
+      x[u][q][0] = x[u][q][1] = 0.0;
+      if (c < nwl) {
+        if (vec && r + 1 < Lt) {
+          const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+          x[u][q][0] = v.x; x[u][q][1] = v.y;
+        } else {
+          if (r < Lt) x[u][q][0] = __ldcg(p);
+          if (r + 1 < Lt) x[u][q][1] = __ldcg(p + a.c_rs);
+        }
+      }
+    }
+  const int ca = tid >> 4, la = tid & 15;              // A1: 16 threads a column
+  double *const A1g = a.mode == 1 ? a.A1 + (size_t)(c0 + ca) * a.a_cs : nullptr;
+  double xa[kKMax / 16];
+#pragma unroll
+  for (int q = 0; q < kKMax / 16; ++q) {
+    const int r = la + 16 * q;
+    xa[q] = (a.mode == 1 && r < k && ca < nwl) ? __ldcg(A1g + (size_t)r * a.a_rs) : 0.0;
+  }
+  // ---- column scales: largest exponent, then the norm ----
+  // high word of |v|, nonzero for every nonzero v
+  auto mag = [](double v) {
+    return ((uint32_t)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u);
+  };
+  uint32_t m0 = 0, m1 = 0, ma = 0;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      m0 = max(m0, mag(x[0][q][e]));
+      m1 = max(m1, mag(x[1][q][e]));
+    }
+#pragma unroll
+  for (int q = 0; q < kKMax / 16; ++q) ma = max(ma, mag(xa[q]));
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
+    m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+  }
+#pragma unroll
+  for (int o = 1; o <= 8; o <<= 1) ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
+  if (t == 0) {
+    red[warp * kCols + g] = m0;
+    red[warp * kCols + g + 8] = m1;
+  }
+  if (la == 0) red[8 * kCols + ca] = ma;
+  __syncthreads();
+  auto col_exp = [&](int c) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int w = 0; w < 9; ++w) m = max(m, red[w * kCols + c]);
+    const int e = m ? (int)(m >> 20) : 1023;           // any scale will do for a column of zeros
+    bad |= (m != 0) & ((e > 1900) | (e < 140));        // far from the ends of the range only
+    return e;
+  };
+  const int e0 = col_exp(g), e1 = col_exp(g + 8), ea = col_exp(ca);
+  // |x| 2^(1022 - emax) < 1 as a float; tiny values go to zero
+  auto rel = [](double v, int emax) {
+    const int h = (int)((uint32_t)__double2hiint(v) & 0x7fffffffu) - ((emax - 126) << 20);
+    return __int_as_float(max(h, 0) << 3);
+  };
+  float n0 = 0.0f, n1 = 0.0f, na = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float f0 = rel(x[0][q][e], e0), f1 = rel(x[1][q][e], e1);
+      n0 = fmaf(f0, f0, n0);
+      n1 = fmaf(f1, f1, n1);
+    }
+#pragma unroll
+  for (int q = 0; q < kKMax / 16; ++q) {
+    const float f = rel(xa[q], ea);
+    na = fmaf(f, f, na);
+  }
+#pragma unroll
+  for (int o = 1; o <= 2; o <<= 1) {
+    n0 += __shfl_xor_sync(0xffffffffu, n0, o);
+    n1 += __shfl_xor_sync(0xffffffffu, n1, o);
+  }
+#pragma unroll
+  for (int o = 1; o <= 8; o <<= 1) na += __shfl_xor_sync(0xffffffffu, na, o);
+  __syncthreads();
+  if (t == 0) {
+    red[warp * kCols + g] = __float_as_uint(n0);
+    red[warp * kCols + g + 8] = __float_as_uint(n1);
+  }
+  if (la == 0) red[8 * kCols + ca] = __float_as_uint(na);
+  __syncthreads();
+  // largest s with norm 2^s <= 2^60.98: norm^2 <= 3.9 * 4^h, s = 60 - h + 1022 - emax
+  auto col_scale = [&](int c, int emax) {
+    float n = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 9; ++w) n += __uint_as_float(red[w * kCols + c]);
+    const int ex = ((__float_as_int(n * (1.0f / 3.9f)) >> 23) & 0xff) - 127;   // floor(log2)
+    return 60 - ((ex + 2) >> 1) + 1022 - emax;
+  };
+  const int s0 = col_scale(g, e0), s1 = col_scale(g + 8, e1), sa = col_scale(ca, ea);
+  long long X[2][4][2];                                // biased by kBias
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      X[0][q][e] = to_fixed<true>(x[0][q][e], s0) + (long long)kBias;
+      X[1][q][e] = to_fixed<true>(x[1][q][e], s1) + (long long)kBias;
+    }
+  if (a.mode == 1) {
+#pragma unroll
+    for (int q = 0; q < kKMax / 16; ++q) {
+      const int r = la + 16 * q;
+      if (r < k) A1s[ca * kKMax + r] = to_fixed<true>(xa[q], sa);
+    }
+  }
+
+  const int nblk = (k + ib - 1) / ib;
+  const uint32_t vbase = saddr(Vd), wbase = saddr(Wd), tbase = saddr(Td);
+  for (int b = 0; b < nblk; ++b) {
+    const int i = a.fwd ? b * ib : (nblk - 1 - b) * ib;
+    const int kb = min(ib, k - i);
+    const int r0 = a.mode == 0 ? i : 0;
+    const int Lr = tt ? min(L, a.tt + i + kb) : L;      // rows this block touches: [r0, Lr)
+    const int wlo = r0 >> 5, whi = (Lr + 31) >> 5;      // warps that hold some of them
+    const bool act = warp >= wlo && warp < whi;
+    const bool two = kb > 16;                           // second half of the 32 reflectors in use
+    // ---- digits of op(T), two pairs (q, q + 1) of one row p each ----
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int idx = tid + u * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
+      unsigned long long y[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        // W2[p] = sum_q op(T)[p, q] W1[q]; op(T) = T^T reads T[q, p]
+        const int row = a.transT ? q + e : p, col = a.transT ? p : q + e;
+        const double v = (row <= col && col < kb) ? __ldcg(a.T + ix(row, i + col, a.ldt)) : 0.0;
+        bad |= ((__double2hiint(v) >> 20) & 0x7ff) >= 1025;
+        y[e] = (unsigned long long)to_fixed<false>(v, 59) + kBias;
+      }
+      const uint32_t off = plane_off(p, q);
+      digits(y[0], y[1], [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Td + d * kPlaneV + off) = w; });
+    }
+    if (act) {
+      // ---- digits of this warp's 32 rows of V ----
+      const int r = 32 * warp + 2 * (lane & 15);
+      const double *const Vg = a.V + ix(r, i, a.ldv);
+      const bool v16 = ((uintptr_t)Vg & 15) == 0 && (a.ldv & 1) == 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (h == 1 && !two) break;
+        double v[8][2];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int p = 16 * h + 2 * u + (lane >> 4);
+          const double *vp = Vg + (size_t)p * a.ldv;
+          // rows [lo, hi) of reflector p are stored; mode 0 adds the unit row lo - 1
+          const int lo = a.mode == 0 ? r0 + p + 1 : 0;
+          const int hi = p < kb ? (tt ? min(Lr, a.tt + i + p + 1) : L) : 0;
+          v[u][0] = v[u][1] = 0.0;
+          if (v16 && r >= lo && r + 1 < hi) {
+            const double2 w = __ldcg(reinterpret_cast<const double2 *>(vp));
+            v[u][0] = w.x; v[u][1] = w.y;
+          } else {
+            if (r >= lo && r < hi) v[u][0] = __ldcg(vp);
+            if (r + 1 >= lo && r + 1 < hi) v[u][1] = __ldcg(vp + 1);
+            if (a.mode == 0 && p < kb) {
+              if (r == lo - 1) v[u][0] = 1.0;
+              if (r + 1 == lo - 1) v[u][1] = 1.0;
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const int p = 16 * h + 2 * u + (lane >> 4);
+          bad |= ((__double2hiint(v[u][0]) & 0x7fffffff) >= 0x3fff0000) |
+                 ((__double2hiint(v[u][1]) & 0x7fffffff) >= 0x3fff0000);       // |v| < 1.9375
+          const unsigned long long y0 = (unsigned long long)to_fixed<false>(v[u][0], 61) + kBias;
+          const unsigned long long y1 = (unsigned long long)to_fixed<false>(v[u][1], 61) + kBias;
+          const uint32_t off = plane_off(p, 2 * (lane & 15));
+          digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Vd + d * kPlaneV + off) = w; });
+        }
+      }
+      __syncwarp();
+      // ---- this warp's share of V^T C, 16 reflectors x 8 columns at a time ----
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint32_t cd[kD][4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          digits((unsigned long long)X[u][q][0], (unsigned long long)X[u][q][1],
+                 [&](int d, uint32_t w) { cd[d][q] = w; });
+#pragma unroll 1
+        for (int mt = 0; mt < (two ? 2 : 1); ++mt) {
+          float acc[kD][4];
+          init_acc(acc);
+          const int p = 16 * mt + (lane & 15);
+#pragma unroll
+          for (int d = 0; d < kD; ++d)
+#pragma unroll
+            for (int kt = 0; kt < 2; ++kt) {
+              uint32_t av[4];
+              ldsm4(vbase + d * kPlaneV + plane_off(p, 16 * kt + 8 * (lane >> 4)), av);
+#pragma unroll
+              for (int j = 0; j < kD - d; ++j)
+                mma(acc[d + j], av[0], av[1], av[2], av[3], cd[j][2 * kt], cd[j][2 * kt + 1]);
+            }
+          long long *wp = Wp + ((size_t)warp * kCols + 8 * u + 2 * t) * kLdWp + 16 * mt + g;
+          wp[0] = recon<47>(acc, 0, bad);
+          wp[kLdWp] = recon<47>(acc, 1, bad);
+          wp[8] = recon<47>(acc, 2, bad);
+          wp[kLdWp + 8] = recon<47>(acc, 3, bad);
+        }
+      }
+    }
+    __syncthreads();
+    // ---- W1 = A1 rows + the warps' shares ----
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int q = tid & 31, c = (tid >> 5) + 8 * u;
+      long long w = 0;
+      if (q < kb) {
+        int top = 0;
+        if (a.mode == 1) {
+          w = A1s[c * kKMax + i + q];
+          top = (int)(w >> 36);
+        }
+        for (int ww = wlo; ww < whi; ++ww) {
+          const long long v = Wp[((size_t)ww * kCols + c) * kLdWp + q];
+          w += v;
+          top += (int)(v >> 36);
+        }
+        bad |= (top > (1 << 26) - (1 << 18)) | (top < -(1 << 26) + (1 << 18));     // |w| < 0.996 * 2^62
+      }
+      W1[c * kLdW1 + q] = w + (long long)kBias;
+    }
+    __syncthreads();
+    // ---- W2 = op(T) W1 (8 reflectors a warp), A1 -= W2, W2's digits ----
+    if (warp < (two ? 4 : 2)) {
+      uint32_t wa[kD][2][4];
+#pragma unroll
+      for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const longlong2 v = *reinterpret_cast<const longlong2 *>(W1 + (g + 8 * (e & 1)) * kLdW1 + 16 * kt + 8 * (e >> 1) + 2 * t);
+          digits((unsigned long long)v.x, (unsigned long long)v.y, [&](int d, uint32_t w) { wa[d][kt][e] = w; });
+        }
+      float acc[kD][4];
+      init_acc(acc);
+#pragma unroll
+      for (int d = 0; d < kD; ++d) {
+        uint32_t bt[4];
+        ldsm4(tbase + d * kPlaneV + plane_off(8 * warp + (lane & 7), 8 * (lane >> 3)), bt);
+#pragma unroll
+        for (int j = 0; j < kD - d; ++j) {
+          mma(acc[d + j], wa[j][0][0], wa[j][0][1], wa[j][0][2], wa[j][0][3], bt[0], bt[1]);
+          mma(acc[d + j], wa[j][1][0], wa[j][1][1], wa[j][1][2], wa[j][1][3], bt[2], bt[3]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int c = g + 8 * u, p = 8 * warp + 2 * t;
+        const long long w0 = recon<49>(acc, 2 * u, bad), w1 = recon<49>(acc, 2 * u + 1, bad);
+        if (a.mode == 1) {
+          long long *ap = A1s + c * kKMax + i + p;
+          if (p < kb) {
+            ap[0] -= w0;
+            bad |= ((uint32_t)(ap[0] >> 32) + 0x40000000u) >> 31;
+          }
+          if (p + 1 < kb) {
+            ap[1] -= w1;
+            bad |= ((uint32_t)(ap[1] >> 32) + 0x40000000u) >> 31;
+          }
+        }
+        const uint32_t off = plane_off(c, p);
+        digits((unsigned long long)w0 + kBias, (unsigned long long)w1 + kBias,
+               [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Wd + d * kPlaneW + off) = w; });
+      }
+    }
+    __syncthreads();
+    // ---- C -= V W2 on this warp's rows, 8 rows at a time ----
+    if (act) {
+      uint32_t wa[kD][2][4];
+#pragma unroll
+      for (int d = 0; d < kD; ++d) {
+        ldsm4(wbase + d * kPlaneW + plane_off(lane & 15, 8 * (lane >> 4)), wa[d][0]);
+        if (two) ldsm4(wbase + d * kPlaneW + plane_off(lane & 15, 16 + 8 * (lane >> 4)), wa[d][1]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float acc[kD][4];
+        init_acc(acc);
+#pragma unroll
+        for (int d = 0; d < kD; ++d) {
+          uint32_t bv[4];
+          ldsm4t(vbase + d * kPlaneV + plane_off(lane, 8 * q), bv);
+#pragma unroll
+          for (int j = 0; j < kD - d; ++j) {
+            mma(acc[d + j], wa[j][0][0], wa[j][0][1], wa[j][0][2], wa[j][0][3], bv[0], bv[1]);
+            if (two) mma(acc[d + j], wa[j][1][0], wa[j][1][1], wa[j][1][2], wa[j][1][3], bv[2], bv[3]);
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            X[u][q][e] -= recon<47>(acc, 2 * u + e, bad);
+            bad |= (int)((uint32_t)(X[u][q][e] >> 32) >> 31);   // left the biased range
+          }
+      }
+      __syncwarp();
+    }
+  }
+  if (__syncthreads_or(bad)) return false;
+
+  // ---- back to FP64: the elements whose value changed ----
+  auto from_fixed = [](long long v, int s) {
+    double d = __ll2double_rn(v);
+    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (s << 20), __double2loint(d));
+  };
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t, s = u ? s1 : s0;
+      double *p = Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs;
+      if (c < nwl) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (r + e < Lt) {
+            double *pe = p + (size_t)e * a.c_rs;
+            const long long v = X[u][q][e] - (long long)kBias;
+            if (v != to_fixed<true>(__ldcg(pe), s)) *pe = from_fixed(v, s);
+          }
+        }
+      }
+    }
+  if (a.mode == 1 && ca < nwl) {
+    for (int r = la; r < k; r += 16) {
+      double *pe = A1g + (size_t)r * a.a_rs;
+      const long long v = A1s[ca * kKMax + r];
+      if (v != to_fixed<true>(__ldcg(pe), sa)) *pe = from_fixed(v, sa);
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+}  // namespace oz
+}  // namespace tqr
