@@ -56,9 +56,16 @@ template <> struct AdjNW<cx<double>> { static constexpr int value = 8; };
 // Dynamic shared memory of the forward and adjoint kernels for element type R:
 // the staged panel, tsqrt block and strip apply at 256 rows, ib = 32.
 template <typename R>
-static size_t adj_smem() {
-  return std::max({kAdjSmem, panel_smem<R>(256, 32, true, true), tsqrt_smem<R>(256, 32, true),
+static size_t adj_smem(bool oz) {
+  return std::max({oz ? oz::kSmem : kAdjSmem, panel_smem<R>(256, 32, true, true), tsqrt_smem<R>(256, 32, true),
                    apply_smem_elems(256, 32, AdjNW<R>::value, true, true, true) * sizeof(R)});
+}
+
+// Double precision: the trailing updates run on the tensor cores
+// (oz_apply.cuh, one CTA per SM) unless the blocks are too small for them.
+template <typename R>
+static bool adj_oz(int n, int ib) {
+  return std::is_same<R, double>::value && oz::covers(1, kAdjNb, n, ib);
 }
 
 struct AdjGeom {
@@ -93,10 +100,10 @@ struct AdjArgs {
 };
 
 // Columns [c0, ncols) of an apply, strip by strip.
-template <typename R>
+template <typename R, bool OZ>
 __device__ void apply_cols(ApplyArgs<R> a, int c0, unsigned char *smem) {
   for (int c = c0; c < a.ncols; c += AdjNW<R>::value) {
-    apply_strip<R, AdjNW<R>::value>(a, c, smem);
+    apply_strip<R, AdjNW<R>::value, OZ>(a, c, smem);
     __syncthreads();
   }
 }
@@ -122,19 +129,19 @@ __device__ ApplyArgs<R> base_args(int ib) {
 // of reflectors starting at column i0 > c then meets W = 0 on column c and
 // leaves it as it is, so each strip [c0, c0 + NW) applies only the blocks
 // starting before c0 + NW: the same values, about half the work of forming Q.
-template <typename R>
+template <typename R, bool OZ>
 __device__ void apply_q(const AdjGeom &g, const R *F, const R *Tw, int trans, R *C, unsigned char *smem,
                         bool ident = false) {
   const int m = g.m, n = g.n, ib = g.ib;
   auto run = [&](ApplyArgs<R> a) {
     if (!ident) {
-      apply_cols<R>(a, 0, smem);
+      apply_cols<R, OZ>(a, 0, smem);
       return;
     }
     constexpr int NW = AdjNW<R>::value;
     for (int c = 0; c < a.ncols; c += NW) {
       a.k = min(n, ((c + NW + ib - 1) / ib) * ib);
-      apply_strip<R, NW>(a, c, smem);
+      apply_strip<R, NW, OZ>(a, c, smem);
       __syncthreads();
     }
   };
@@ -166,7 +173,7 @@ __device__ void apply_q(const AdjGeom &g, const R *F, const R *Tw, int trans, R 
 
 // Flat-tree tile QR of one problem in place; T blocks to Tw (tile t's at
 // Tw + t * 32 * n, ld ib), tau to tau (tile t's at tau + t * n).
-template <typename R>
+template <typename R, bool OZ>
 __device__ void factor_one(const AdjGeom &g, R *A, R *tau, R *Tw, unsigned char *smem) {
   const int m = g.m, n = g.n, ib = g.ib, lda = m;
   const int L0 = g.rows(0);
@@ -178,7 +185,7 @@ __device__ void factor_one(const AdjGeom &g, R *A, R *tau, R *Tw, unsigned char 
     a.C = A + i0; a.c_cs = lda; a.ncols = n;
     a.V = A + ix(i0, i0, lda); a.ldv = lda;
     a.T = Tw + ix(0, i0, ib); a.ldt = ib;
-    apply_cols<R>(a, i0 + sb, smem);
+    apply_cols<R, OZ>(a, i0 + sb, smem);
   }
   for (int t = 1; t < g.MT; ++t) {
     R *At = A + (size_t)t * kAdjNb;
@@ -198,7 +205,7 @@ __device__ void factor_one(const AdjGeom &g, R *A, R *tau, R *Tw, unsigned char 
       a.A1 = A + i0; a.a_cs = lda;
       a.V = At + ix(0, i0, lda); a.ldv = lda;
       a.T = Tt + ix(0, i0, ib); a.ldt = ib;
-      apply_cols<R>(a, i0 + sb, smem);
+      apply_cols<R, OZ>(a, i0 + sb, smem);
     }
   }
 }
@@ -322,13 +329,13 @@ __global__ void __launch_bounds__(TQR_THREADS) k_solve_rt(AdjGeom g, const R *F,
   solve_rt<R>(g.rows(t), g.n, F + off, g.m, Abar + off + (size_t)t * kAdjNb, g.m, smem_raw);
 }
 
-template <typename R>
+template <typename R, bool OZ>
 __device__ void forward_one(const AdjArgs<R> &a, int p, R *Tw, unsigned char *smem) {
   const AdjGeom &g = a.g;
   const int m = g.m, n = g.n;
   R *A = a.F + (size_t)p * m * n;
   R *tau = a.tau + (size_t)p * g.MT * n;
-  factor_one<R>(g, A, tau, Tw, smem);
+  factor_one<R, OZ>(g, A, tau, Tw, smem);
   __syncthreads();
   R *Rp = a.Rout + (size_t)p * n * n;
   R *Qp = a.Q + (size_t)p * m * n;
@@ -341,10 +348,10 @@ __device__ void forward_one(const AdjArgs<R> &a, int p, R *Tw, unsigned char *sm
     Qp[idx] = (r == c) ? R(1) : R(0);
   }
   __syncthreads();
-  apply_q<R>(g, A, Tw, 0, Qp, smem, true);
+  apply_q<R, OZ>(g, A, Tw, 0, Qp, smem, true);
 }
 
-template <typename R>
+template <typename R, bool OZ>
 __device__ void backward_one(const AdjArgs<R> &a, int p, R *Tw, R *Ms, unsigned char *smem) {
   const AdjGeom &g = a.g;
   const int m = g.m, n = g.n;
@@ -358,7 +365,7 @@ __device__ void backward_one(const AdjArgs<R> &a, int p, R *Tw, R *Ms, unsigned 
   // W := Q_full^T Qbar; its first n rows are Q^T Qbar
   for (size_t idx = tid; idx < (size_t)m * n; idx += TQR_THREADS) W[idx] = Qb[idx];
   __syncthreads();
-  apply_q<R>(g, F, Tw, 1, W, smem);
+  apply_q<R, OZ>(g, F, Tw, 1, W, smem);
   // Ms (lower) = R Rbar^H - (Q^H Qbar)^H
   for (int idx = tid; idx < n * n; idx += TQR_THREADS) {
     const int i = idx % n, j = idx / n;
@@ -382,15 +389,15 @@ __device__ void backward_one(const AdjArgs<R> &a, int p, R *Tw, R *Ms, unsigned 
     W[idx] = v;
   }
   __syncthreads();
-  apply_q<R>(g, F, Tw, 0, W, smem);
+  apply_q<R, OZ>(g, F, Tw, 0, W, smem);
   // Y = Qbar + Q copyltu(M);  Abar = Y R^-T
   for (size_t idx = tid; idx < (size_t)m * n; idx += TQR_THREADS) W[idx] += Qb[idx];
   __syncthreads();
   // Abar = Y R^-T follows in k_solve_rt
 }
 
-template <typename R>
-__global__ void __launch_bounds__(TQR_THREADS, 2) k_qr_fwd(const AdjArgs<R> a) {
+template <typename R, bool OZ>
+__global__ void __launch_bounds__(TQR_THREADS, OZ ? 1 : 2) k_qr_fwd(const AdjArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_p;
   R *Tw = a.scratch + (size_t)blockIdx.x * adj_scratch_elems<R>(a.g);
@@ -400,13 +407,13 @@ __global__ void __launch_bounds__(TQR_THREADS, 2) k_qr_fwd(const AdjArgs<R> a) {
     const int p = s_p;
     __syncthreads();
     if (p >= a.batch) break;
-    forward_one<R>(a, p, Tw, smem_raw);
+    forward_one<R, OZ>(a, p, Tw, smem_raw);
     __syncthreads();
   }
 }
 
-template <typename R>
-__global__ void __launch_bounds__(TQR_THREADS, 2) k_qr_bwd(const AdjArgs<R> a) {
+template <typename R, bool OZ>
+__global__ void __launch_bounds__(TQR_THREADS, OZ ? 1 : 2) k_qr_bwd(const AdjArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_p;
   R *Tw = a.scratch + (size_t)blockIdx.x * adj_scratch_elems<R>(a.g);
@@ -417,7 +424,7 @@ __global__ void __launch_bounds__(TQR_THREADS, 2) k_qr_bwd(const AdjArgs<R> a) {
     const int p = s_p;
     __syncthreads();
     if (p >= a.batch) break;
-    backward_one<R>(a, p, Tw, Ms, smem_raw);
+    backward_one<R, OZ>(a, p, Tw, Ms, smem_raw);
     __syncthreads();
   }
 }
@@ -427,28 +434,28 @@ __global__ void k_adj_reset(AdjHeader *h) {
 }
 
 static std::mutex g_adj_mu;
-static int g_adj_grid[4][2][64];      // [element type][fwd/bwd][device]
+static int g_adj_grid[2][4][2][64];   // [tensor cores][element type][fwd/bwd][device]
 
 template <typename R> constexpr int adj_slot() {
   return std::is_same<R, double>::value ? 0 : std::is_same<R, float>::value ? 1 : std::is_same<R, cx<double>>::value ? 2 : 3;
 }
 
-template <typename R, bool FWD>
+template <typename R, bool FWD, bool OZ>
 static int adj_grid(int *grid) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
   if (dev >= 64) return (int)cudaErrorInvalidDevice;
   std::lock_guard<std::mutex> l(g_adj_mu);
-  int &gsz = g_adj_grid[adj_slot<R>()][FWD ? 0 : 1][dev];
+  int &gsz = g_adj_grid[OZ][adj_slot<R>()][FWD ? 0 : 1][dev];
   if (gsz == 0) {
     int sms = 0, per = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-    auto kern = FWD ? k_qr_fwd<R> : k_qr_bwd<R>;
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem<R>())) !=
+    auto kern = FWD ? k_qr_fwd<R, OZ> : k_qr_bwd<R, OZ>;
+    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)adj_smem<R>(OZ))) !=
         cudaSuccess)
       return (int)e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, TQR_THREADS, adj_smem<R>())) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, TQR_THREADS, adj_smem<R>(OZ))) != cudaSuccess)
       return (int)e;
     gsz = sms * std::max(per, 1);
   }
@@ -468,8 +475,16 @@ static int adj_worksize(int m, int n, int ib, size_t *bytes, int *grid_out) {
   AdjGeom g;
   if (!adj_geom(m, n, ib, &g)) return -1;
   int gf = 0, gb = 0, rc;
-  if ((rc = adj_grid<R, true>(&gf)) != 0) return rc;
-  if ((rc = adj_grid<R, false>(&gb)) != 0) return rc;
+  if constexpr (std::is_same<R, double>::value) {
+    if (adj_oz<R>(n, ib)) {
+      if ((rc = adj_grid<R, true, true>(&gf)) != 0) return rc;
+      if ((rc = adj_grid<R, false, true>(&gb)) != 0) return rc;
+    }
+  }
+  if (gf == 0) {
+    if ((rc = adj_grid<R, true, false>(&gf)) != 0) return rc;
+    if ((rc = adj_grid<R, false, false>(&gb)) != 0) return rc;
+  }
   const int grid = std::max(gf, gb);
   *bytes = sizeof(AdjHeader) + sizeof(R) * adj_scratch_elems<R>(g) * (size_t)grid;
   if (grid_out) *grid_out = grid;
@@ -507,12 +522,15 @@ static int adj_launch(int batch, int m, int n, int ib, R *F, R *tau, R *Q, R *Ro
   k_adj_reset<<<1, 32, 0, st>>>(a.hdr);
   count_launch();
   const int gl = std::min(grid, batch);
-  if (FWD) {
-    k_qr_fwd<R><<<gl, TQR_THREADS, adj_smem<R>(), st>>>(a);
-    count_launch();
-  } else {
-    k_qr_bwd<R><<<gl, TQR_THREADS, adj_smem<R>(), st>>>(a);
-    count_launch();
+  auto kern = FWD ? k_qr_fwd<R, false> : k_qr_bwd<R, false>;
+  bool oz = false;
+  if constexpr (std::is_same<R, double>::value) {
+    oz = adj_oz<R>(n, ib);
+    if (oz) kern = FWD ? k_qr_fwd<R, true> : k_qr_bwd<R, true>;
+  }
+  kern<<<gl, TQR_THREADS, adj_smem<R>(oz), st>>>(a);
+  count_launch();
+  if (!FWD) {
     const size_t sm = sizeof(R) * ((size_t)kAdjNb * SolveBw<R>::value + SolveBw<R>::value);
     cudaError_t e = cudaSuccess;
     if (sm > 48 * 1024)

@@ -135,7 +135,7 @@ __device__ ApplyArgs<R> tree_args(int mode, int L, int k, int ib, int trans) {
 // One step of the tree factorisation on top tile i (and partner i + op.s for
 // the pair ops), strip y; shared by the stream driver and the persistent
 // task-graph kernel.
-template <typename R>
+template <typename R, bool OZ>
 __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, unsigned char *smem) {
   const int k = op.k, ib = g.ib, nk = g.cols(k);
   const int mi = g.rows(i);
@@ -159,7 +159,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
       a.C = Aik + c; a.c_cs = g.lda; a.ncols = nk;
       a.V = Aik + ix(c, c, g.lda); a.ldv = g.lda;
       a.T = g.ttile(g.T, i, k) + ix(0, c, g.ldt); a.ldt = g.ldt;
-      apply_strip<R, TreeNW<R>::value>(a, c0, smem);
+      apply_strip<R, TreeNW<R>::value, OZ>(a, c0, smem);
       return;
     }
     case OP_GE_TRAIL: {
@@ -169,7 +169,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
       a.C = C; a.c_cs = ld; a.ncols = ncols;
       a.V = Aik; a.ldv = g.lda;
       a.T = g.ttile(g.T, i, k); a.ldt = g.ldt;
-      apply_strip<R, TreeNW<R>::value>(a, c0, smem);
+      apply_strip<R, TreeNW<R>::value, OZ>(a, c0, smem);
       return;
     }
     default:
@@ -202,7 +202,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
       a.V = Apk + ix(0, c, g.lda); a.ldv = g.lda;
       a.T = g.ttile(g.T2, p, k) + ix(0, c, g.ldt); a.ldt = g.ldt;
       a.tt = op.ts ? -1 : c;
-      apply_strip<R, TreeNW<R>::value>(a, c0, smem);
+      apply_strip<R, TreeNW<R>::value, OZ>(a, c0, smem);
       return;
     }
     case OP_PR_TRAIL: {
@@ -216,7 +216,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
       a.V = Apk; a.ldv = g.lda;
       a.T = g.ttile(g.T2, p, k); a.ldt = g.ldt;
       a.tt = op.ts ? -1 : 0;
-      apply_strip<R, TreeNW<R>::value>(a, c0, smem);
+      apply_strip<R, TreeNW<R>::value, OZ>(a, c0, smem);
       return;
     }
     default:
@@ -224,18 +224,41 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
   }
 }
 
+// Double precision: whether the strip updates run on the tensor cores
+// (oz_apply.cuh; OZ below), which takes one CTA per SM.
 template <typename R>
-__global__ void __launch_bounds__(TQR_THREADS, 2) k_tree(const TreeGeom<R> g, const TreeOp op) {
+static bool tree_oz(int nb, int ib) {
+  return std::is_same<R, double>::value && oz::covers(1, nb, nb, ib);
+}
+
+template <typename R, bool OZ>
+__global__ void __launch_bounds__(TQR_THREADS, OZ ? 1 : 2) k_tree(const TreeGeom<R> g, const TreeOp op) {
   extern __shared__ __align__(16) unsigned char smem[];
-  tree_task<R>(g, op, op.i0 + blockIdx.x * op.istep, blockIdx.y, smem);
+  tree_task<R, OZ>(g, op, op.i0 + blockIdx.x * op.istep, blockIdx.y, smem);
 }
 
 template <typename R>
 static cudaError_t tree_launch(const TreeGeom<R> &g, const TreeOp &op, int ntask, int ny, cudaStream_t st) {
   if (ntask <= 0 || ny <= 0) return cudaSuccess;
-  k_tree<R><<<dim3(ntask, ny), TQR_THREADS, tree_smem<R>(), st>>>(g, op);
+  if constexpr (std::is_same<R, double>::value) {
+    if (tree_oz<R>(g.nb, g.ib)) {
+      k_tree<R, true><<<dim3(ntask, ny), TQR_THREADS, oz::kSmem, st>>>(g, op);
+      count_launch();
+      return cudaGetLastError();
+    }
+  }
+  k_tree<R, false><<<dim3(ntask, ny), TQR_THREADS, tree_smem<R>(), st>>>(g, op);
   count_launch();
   return cudaGetLastError();
+}
+
+template <typename R>
+static cudaError_t tree_kernel_attr() {
+  if constexpr (std::is_same<R, double>::value) {
+    cudaError_t e = cudaFuncSetAttribute(k_tree<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::kSmem);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaFuncSetAttribute(k_tree<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem<R>());
 }
 
 template <typename R>
@@ -265,7 +288,7 @@ static inline int tree_nlead(int k, int MTt, int grp) { return (MTt - k + grp - 
 
 template <typename R>
 static cudaError_t tree_factor(const TreeGeom<R> &g, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_tree<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem<R>());
+  cudaError_t e = tree_kernel_attr<R>();
   if (e != cudaSuccess) return e;
   constexpr int nw = TreeNW<R>::value;
   const int ib = g.ib, G = g.grp;
@@ -324,7 +347,7 @@ static cudaError_t tree_factor(const TreeGeom<R> &g, cudaStream_t st) {
 // B := Q^T B (trans 0) or Q B (trans 1) through the stored tree factors.
 template <typename R>
 static cudaError_t tree_apply_q(const TreeGeom<R> &g, int trans, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_tree<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tree_smem<R>());
+  cudaError_t e = tree_kernel_attr<R>();
   if (e != cudaSuccess) return e;
   constexpr int nw = TreeNW<R>::value;
   const int ny = (g.nrhs + nw - 1) / nw, G = g.grp;
@@ -533,9 +556,10 @@ __device__ __forceinline__ unsigned long long tdag_ns() {
 }
 
 // TC: this instantiation owns the SM's TMEM and runs the tensor-core chunk
-// tasks (FP32, one CTA per SM); the other instantiations never meet one.
-template <typename R, bool TC>
-__global__ void __launch_bounds__(TQR_THREADS, TC ? 1 : 2) k_tree_dag(const __grid_constant__ TDagArgs<R> a) {
+// tasks (FP32, one CTA per SM); the other instantiations never meet one.  OZ:
+// FP64 strips on the tensor cores.
+template <typename R, bool TC, bool OZ>
+__global__ void __launch_bounds__(TQR_THREADS, TC || OZ ? 1 : 2) k_tree_dag(const __grid_constant__ TDagArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_it, s_err;
   __shared__ __align__(8) uint64_t s_bars[tc::kBars];
@@ -681,10 +705,10 @@ __global__ void __launch_bounds__(TQR_THREADS, TC ? 1 : 2) k_tree_dag(const __gr
       } else if (a.D && (op.type == OP_GE_PANEL || op.type == OP_PR_PANEL)) {
         tree_panel_f64(a, op, it.i, smem);
       } else {
-        tree_task<R>(a.g, op, it.i, it.y, smem);
+        tree_task<R, OZ>(a.g, op, it.i, it.y, smem);
       }
     } else {
-      tree_task<R>(a.g, op, it.i, it.y, smem);
+      tree_task<R, OZ>(a.g, op, it.i, it.y, smem);
     }
     if (!ok) {
       if (tid == 0 && atomicCAS(&a.hdr->error, 0, 3) == 0) a.hdr->err_item = idx;
@@ -1078,21 +1102,21 @@ static size_t tree_work_bytes(TreeShape sh) {
   return b;
 }
 
-template <typename R, bool TC>
+template <typename R, bool TC, bool OZ = false>
 static cudaError_t tree_dag_launch(const TDagArgs<R> &a, size_t sm, cudaStream_t st) {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_tree_dag<R, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
+  if ((e = cudaFuncSetAttribute(k_tree_dag<R, TC, OZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
       cudaSuccess)
     return e;
   int dev = 0, sms = 0, per_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tree_dag<R, TC>, TQR_THREADS, sm)) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tree_dag<R, TC, OZ>, TQR_THREADS, sm)) !=
       cudaSuccess)
     return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int grid = std::min(sms * per_sm, a.nitems);
-  k_tree_dag<R, TC><<<grid, TQR_THREADS, sm, st>>>(a);
+  k_tree_dag<R, TC, OZ><<<grid, TQR_THREADS, sm, st>>>(a);
   count_launch();
   return cudaGetLastError();
 }
@@ -1167,6 +1191,12 @@ static int tree_geqrf_dag_impl(int m, int n, int nb, int ib, R *A, int lda, R *T
   if constexpr (std::is_same<R, float>::value) {
     if (sh.tc) {
       e = tree_dag_launch<R, true>(a, std::max({sm, tc::kSmem, tc::wy::kSmem}), st);
+      return e == cudaSuccess ? 0 : (int)e;
+    }
+  }
+  if constexpr (std::is_same<R, double>::value) {
+    if (tree_oz<R>(nb, ib)) {
+      e = tree_dag_launch<R, false, true>(a, std::max(sm, oz::kSmem), st);
       return e == cudaSuccess ? 0 : (int)e;
     }
   }
