@@ -152,7 +152,9 @@ __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_r
   const int nwl = min(NW, a.ncols - c0);
   if (nwl <= 0) return;
   if constexpr (VEC && std::is_same<R, double>::value && NW <= oz::kCols) {
-    if (oz::covers(a.mode, a.L, a.k, a.ib) && oz::strip<0>(a, c0, nwl, smem_raw)) return;
+    if (oz::covers(a.mode, a.L, a.k, a.ib) && 
+        oz::strip<1>(a, c0, nwl, smem_raw, reinterpret_cast<long long *>(smem_raw + oz::kOffA1)))
+      return;
   }
   const int L = a.L, ib = a.ib;
   const int ldw = ib;

@@ -13,10 +13,10 @@
 // accumulation is exact, whatever its order.
 //
 // Number format.  Column c of [A1; C] is held as 64-bit fixed point with its
-// own power-of-two scale 2^s: s is the largest with ||column|| 2^s <= 2^60.98.
+// own power-of-two scale 2^s: s is the largest with ||column|| 2^s <= 2^60.9.
 // An orthogonal update keeps that norm, |W| <= 2 ||column||, so nothing leaves
-// the 62-bit range the digits cover; V (|v| < 1.94) is scaled by 2^61 and T
-// (|t| < 4) by 2^59.  A strip that is not such an update (an infinity or NaN,
+// the 62-bit range the digits cover; V (|v| < 1.93) is scaled by 2^61 and T
+// (|t| < 3.87) by 2^60.  A strip that is not such an update (an infinity or NaN,
 // exponents near the ends of the range, a V or T beyond those bounds, a sum
 // that overflows) is detected before anything is written and the caller runs
 // the DFMA path on it.  An element whose fixed-point value the update did not
@@ -24,9 +24,9 @@
 //
 // Accuracy.  With c the column's root mean square over r rows, the unit of
 // the fixed point is 2^-61 sqrt(r) c; the dropped digit products (i + j > 6)
-// add about 2^3.7 units to W and 2^2.2 to C, where the FP64 sums they replace
-// round 256 and 32 times at 2^-53: measured against 64-bit references the
-// results are as close or closer.
+// add about 2^2 units to W and to C, where the FP64 sums they replace round
+// 256 and 32 times at 2^-53.  Against extended precision a 256-row tsmqr is
+// 3.0e-16 off, normwise, with the FP64 loops 4.4e-16.
 //
 // Layout.  Warp w owns rows [32 w, 32 w + 32) of the strip in registers, as
 // the accumulator fragment of (V W)^T: lane (g, t) = (lane / 4, lane % 4)
@@ -52,23 +52,26 @@ template <typename R> struct ApplyArgs;
 
 namespace oz {
 
-constexpr int kCols = 16;              // strip columns
+constexpr int kCols = 16;              // strip columns of a group of eight warps
 constexpr int kRowsMax = 256;          // region rows: 32 per warp
 constexpr int kIbMax = 32;
-constexpr int kKMax = 256;             // reflectors of a mode 1 apply (A1 rows kept in shared memory)
+constexpr int kKMax = 256;             // reflectors of a mode 1 apply (A1 rows kept until the end)
 constexpr int kD = 7;                  // digits
-constexpr uint32_t kPlaneV = 32 * 64;  // one digit plane of a warp's V: 32 reflectors x 32 rows
+constexpr uint32_t kPlaneV = 32 * 64;  // one digit plane of 32 rows of V: 32 reflectors x 32 rows
 constexpr uint32_t kWarpV = kD * kPlaneV;
 constexpr uint32_t kPlaneW = 16 * 64;
 constexpr int kLdWp = 36, kLdW1 = 40;
-// shared memory: V digits | T digits | W digits | partial W | W | A1 | reductions
+// shared memory: V digits | T digits, then per group: W digits | partial W |
+// W | reductions, then (one group) A1
 constexpr size_t kOffT = 8 * (size_t)kWarpV;
-constexpr size_t kOffW = kOffT + kD * (size_t)kPlaneV;
-constexpr size_t kOffWp = kOffW + kD * (size_t)kPlaneW;
-constexpr size_t kOffW1 = kOffWp + sizeof(long long) * 8 * kCols * kLdWp;
-constexpr size_t kOffA1 = kOffW1 + sizeof(long long) * kCols * kLdW1;
-constexpr size_t kOffRed = kOffA1 + sizeof(long long) * kCols * kKMax;
-constexpr size_t kSmem = kOffRed + sizeof(uint32_t) * kCols * 9;
+constexpr size_t kOffG = kOffT + kD * (size_t)kPlaneV;
+constexpr size_t kGrpW1 = kD * (size_t)kPlaneW;
+constexpr size_t kGrpWp = kGrpW1 + sizeof(long long) * kCols * kLdW1;
+constexpr size_t kGrpRed = kGrpWp + sizeof(long long) * 8 * kCols * kLdWp;
+constexpr size_t kGrpSh = kGrpRed + sizeof(uint32_t) * kCols * 9;
+constexpr size_t kGrp = kGrpSh + sizeof(uint32_t) * 16;
+constexpr size_t kOffA1 = kOffG + kGrp;
+constexpr size_t kSmem = kOffA1 + sizeof(long long) * kCols * kKMax;
 static_assert(kSmem <= TQR_SMEM_MAX, "one CTA's shared memory");
 
 // 256 in every digit: x + kBias has the digits of x plus 256, without carries
@@ -79,7 +82,7 @@ __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cv
 
 __device__ __forceinline__ void mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                     uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
@@ -88,19 +91,21 @@ __device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
-__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+
+__device__ __forceinline__ void ldsm2(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm2t(uint32_t addr, uint32_t (&r)[2]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(addr) : "memory");
 }
 
 // x 2^s as an integer, rounded to nearest (RND) or towards zero; the caller
-// has checked that |x| 2^s < 2^62.
+// sees to |x| 2^s < 2^62 (larger and non-finite values give garbage).
 template <bool RND>
 __device__ __forceinline__ long long to_fixed(double x, int s) {
   const uint32_t hi = __double2hiint(x), lo = __double2loint(x);
-  const int e = (int)((hi >> 20) & 0x7ff);
   unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
-  unsigned int t = (unsigned int)(1085 - s - e);      // m 2^-t is |x| 2^s; zeros and subnormals shift out
+  const int t = (1085 - s) - (int)((hi >> 20) & 0x7ff);   // m 2^-t is |x| 2^s; zeros and subnormals shift out
   if (RND) {
     // shr clamps the shift count, so a long shift gives zero
     asm("shr.u64 %0, %1, %2;" : "=l"(m) : "l"(m), "r"(t - 1));
@@ -110,6 +115,16 @@ __device__ __forceinline__ long long to_fixed(double x, int s) {
   }
   const long long sg = (long long)((int)hi >> 31);
   return ((long long)m ^ sg) - sg;
+}
+// the same, with the largest high word of |x| collected for a bound check
+__device__ __forceinline__ long long to_fixed_max(double x, int s, uint32_t &hmax) {
+  hmax = max(hmax, (uint32_t)__double2hiint(x) & 0x7fffffffu);
+  return to_fixed<false>(x, s);
+}
+
+__device__ __forceinline__ double from_fixed(long long v, int s) {
+  const double d = __ll2double_rn(v);
+  return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (s << 20), __double2loint(d));
 }
 
 // Digit J (0 = lowest) of two biased fixed-point values as an f16 pair.
@@ -151,91 +166,141 @@ __device__ __forceinline__ void init_acc(F (&acc)[kD][4]) {
     for (int e = 0; e < 4; ++e) acc[d][e] = d < 2 ? kMagic : 0.0f;
 }
 
-// sum_d acc[d] 2^(SH - 9 d), rounded once below the unit; sets bad when the
-// value leaves (-2^62, 2^62).  Diagonals 0 and 1 (|sum| <= 2^22) were
-// accumulated on top of kMagic, so their integers are read from the bits.
+// sum_d acc[d][e] 2^(SH - 9 d), rounded once below the unit.  Diagonals 0 and
+// 1 (|sum| <= 2^22) were accumulated on top of kMagic, so their integers are
+// the low bits.  big collects acc[0] + 2^(62 - SH): while that stays in
+// [0, 2^(63 - SH)) the value is below 2^63 in magnitude (the other diagonals
+// add less than 2^62).
 template <int SH>
-__device__ __forceinline__ long long recon(const float (&acc)[kD][4], int e, int &bad) {
-  const int i0 = __float_as_int(acc[0][e]) - 0x4B400000, i1 = __float_as_int(acc[1][e]) - 0x4B400000;
+__device__ __forceinline__ long long recon(const float (&acc)[kD][4], int e, uint32_t &big) {
+  const int r0 = __float_as_int(acc[0][e]), r1 = __float_as_int(acc[1][e]);
   const int i2 = __float2int_rn(acc[2][e]), i3 = __float2int_rn(acc[3][e]), i4 = __float2int_rn(acc[4][e]);
   const int i5 = __float2int_rn(fmaf(acc[5][e], (float)(1 << (SH - 45)), acc[6][e] * (1.0f / (float)(1 << (54 - SH)))));
+  constexpr uint32_t base = 0u - (0x4B400000u << (SH - 32)) - (0x4B400000u << (SH - 41));
   long long r = (long long)i5;
   r += (long long)i4 * (1ll << (SH - 36));
   r += (long long)i3 * (1ll << (SH - 27));
   r += (long long)i2 * (1ll << (SH - 18));
-  r += (long long)((i0 << (SH - 32)) + (i1 << (SH - 41))) << 32;
-  // |value| / 2^SH is within 26 / 512 of |i0 + i1 / 512|
-  const int top = i0 + (i1 >> 9);
-  constexpr int lim = (int)((1ll << (62 - SH)) * 0.99);
-  bad |= (top > lim) | (top < -lim);
-  return r;
+  const uint32_t hi = (uint32_t)r0 * (1u << (SH - 32)) + ((uint32_t)r1 * (1u << (SH - 41)) + base);
+  big |= ((uint32_t)r0 - (0x4B400000u - (1u << (62 - SH)))) << (SH - 47);
+  return r + (long long)((unsigned long long)hi << 32);
 }
+constexpr uint32_t kBig = 0xffff0000u;   // bits of big that mean an overflow
 
 // Byte offset of 16-bit element (row, k), k even, in a plane of 64-byte rows.
 __device__ __forceinline__ uint32_t plane_off(int row, int k) {
   return (uint32_t)row * 64u + (uint32_t)((((k >> 3) ^ (row >> 1)) & 3) << 4) + (uint32_t)((k & 7) * 2);
 }
 
-// Whether the arguments are ones strip() covers; a property of the call, not
-// of the strip, so every driver of the same update takes the same path.
-// Below 48 rows or 12 reflectors the DFMA loops are the faster ones (the
-// fixed cost of a block is a few thousand clocks; see the figures in
-// apply_strip).
+// Whether strip() takes a call: a property of the call, not of the strip, so
+// that every driver of the same update takes the same path.  The lines are
+// where the two paths cross.  One block of 32 reflectors on 16 columns costs
+// strip() 23 us whatever the rows (10 us of them to bring the strip into
+// fixed point and back); the DFMA loops take 64 us at 256 rows in a task graph,
+// 29 us where a narrow stand-alone call spreads over one-column strips (23 at
+// 192 rows, 19 at 128).  Four blocks: 45 us against 38 at 32 rows, 46 at 64,
+// 101 at 256 (stand-alone, 16 columns).
 __host__ __device__ inline bool covers(int mode, int L, int k, int ib) {
-  return ib <= kIbMax && L <= kRowsMax && (mode == 0 || k <= kKMax) && (ib < k ? ib : k) >= 8 && L >= 32;
+  return ib <= kIbMax && L <= kRowsMax && (mode == 0 || k <= kKMax) &&
+         L * (ib < k ? ib : k) >= (k > ib ? 32 * 32 * 2 : 128 * 32);
 }
 
-// Applies to the strip of columns [c0, c0 + nwl).  False: the strip needs the
-// DFMA path; nothing has been written.  All threads get the same answer.
-template <int kUnused>
-__device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+// Rows r, r + 1 of reflectors p, p + 2, p + 4, p + 6 of a block at column i:
+// the stored entries, with mode 0's unit diagonal and the zeros above it.
+// whole: all of them are stored entries, 16-byte aligned.
+__device__ __forceinline__ void load_v(const ApplyArgs<double> &a, const double *Vg, bool whole, int r, int p, int kb,
+                                       int i, int Lr, bool tt, double (&v)[4][2]) {
+  if (whole) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double2 w = __ldcg(reinterpret_cast<const double2 *>(Vg + (size_t)(p + 2 * u) * a.ldv));
+      v[u][0] = w.x; v[u][1] = w.y;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int pu = p + 2 * u;
+      const int lo = a.mode == 0 ? i + pu + 1 : 0;
+      const int hi = pu < kb ? (tt ? min(Lr, a.tt + i + pu + 1) : a.L) : 0;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        v[u][e] = (r + e >= lo && r + e < hi) ? __ldcg(Vg + e + (size_t)pu * a.ldv) : 0.0;
+        if (a.mode == 0 && pu < kb && r + e == lo - 1) v[u][e] = 1.0;
+      }
+    }
+  }
+}
+
+// Applies to the strip of columns [c0, c0 + nwl), nwl <= 16 G, with G groups
+// of 256 threads, 16 columns each, sharing V's and T's digits.  a1buf: 16 G x
+// kKMax values (mode 1).  False: the strip needs the DFMA path; nothing has
+// been written.  All threads get the same answer.
+template <int G>
+__device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem,
+                                   long long *a1buf) {
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int grp = G == 1 ? 0 : tid >> 8, gtid = tid & 255, warp = gtid >> 5;
   const int L = a.L, ib = a.ib, k = a.k;
-  unsigned char *Vd = smem + (size_t)warp * kWarpV;
-  unsigned char *Td = smem + kOffT, *Wd = smem + kOffW;
-  long long *Wp = reinterpret_cast<long long *>(smem + kOffWp);
-  long long *W1 = reinterpret_cast<long long *>(smem + kOffW1);
-  long long *A1s = reinterpret_cast<long long *>(smem + kOffA1);
-  uint32_t *red = reinterpret_cast<uint32_t *>(smem + kOffRed);   // [warp 0..7, A1][column]
+  unsigned char *const Vd = smem + (size_t)warp * kWarpV, *const Td = smem + kOffT;
+  unsigned char *const gs = smem + kOffG + grp * kGrp, *const Wd = gs;
+  long long *const W1 = reinterpret_cast<long long *>(gs + kGrpW1);
+  long long *const Wp = reinterpret_cast<long long *>(gs + kGrpWp);
+  uint32_t *const red = reinterpret_cast<uint32_t *>(gs + kGrpRed);   // [warp 0..7, A1][column]
+  uint32_t *const shw = reinterpret_cast<uint32_t *>(gs + kGrpSh);    // per warp: V^T C's share is scaled by 2^shw
+  long long *const A1s = a1buf + (size_t)grp * kCols * kKMax;
+  c0 += kCols * grp;
+  nwl = min(kCols, nwl - kCols * grp);
   const bool tt = a.mode == 1 && a.tt >= 0;
   const int Lt = tt ? min(L, a.tt + k) : L;            // rows any reflector touches
   int bad = 0;
+  uint32_t big = 0, vmax = 0, tmax = 0;
 
   // ---- the strip, and A1's rows, from global memory ----
   double *const Cg = a.C + (size_t)c0 * a.c_cs;
   const bool vec = a.c_rs == 1 && ((uintptr_t)Cg & 15) == 0 && (a.c_cs & 1) == 0;
-  double x[2][4][2];
+  // this lane's elements of the strip: 16-byte loads, all in flight, where the
+  // warp's 32 x 16 block is whole and aligned
+  const bool whole = vec && nwl == kCols && 32 * warp + 32 <= Lt;
+  auto load_c = [&](double (&x)[2][4][2]) {
+    if (whole) {
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+      for (int u = 0; u < 2; ++u)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t;
-      const double *p = Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs;
-      x[u][q][0] = x[u][q][1] = 0.0;
-      if (c < nwl) {
-        if (vec && r + 1 < Lt) {
-          const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+        for (int q = 0; q < 4; ++q) {
+          const double2 v = __ldcg(reinterpret_cast<const double2 *>(Cg + 32 * warp + 8 * q + 2 * t +
+                                                                     (size_t)(g + 8 * u) * a.c_cs));
           x[u][q][0] = v.x; x[u][q][1] = v.y;
-        } else {
-          if (r < Lt) x[u][q][0] = __ldcg(p);
-          if (r + 1 < Lt) x[u][q][1] = __ldcg(p + a.c_rs);
         }
-      }
-    }
-  const int ca = tid >> 4, la = tid & 15;              // A1: 16 threads a column
-  double *const A1g = a.mode == 1 ? a.A1 + (size_t)(c0 + ca) * a.a_cs : nullptr;
-  double xa[kKMax / 16];
+    } else {
 #pragma unroll
-  for (int q = 0; q < kKMax / 16; ++q) {
-    const int r = la + 16 * q;
-    xa[q] = (a.mode == 1 && r < k && ca < nwl) ? __ldcg(A1g + (size_t)r * a.a_rs) : 0.0;
-  }
-  // ---- column scales: largest exponent, then the norm ----
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t + e;
+            x[u][q][e] = (c < nwl && r < Lt) ? __ldcg(Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs) : 0.0;
+          }
+    }
+  };
+  double x[2][4][2];
+  load_c(x);
   // high word of |v|, nonzero for every nonzero v
   auto mag = [](double v) {
     return ((uint32_t)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u);
   };
+  const int ca = gtid >> 4, la = gtid & 15;            // A1: 16 threads a column
+  double *const A1g = a.mode == 1 ? a.A1 + (size_t)(c0 + ca) * a.a_cs : nullptr;
+  const int ka = a.mode == 1 && ca < nwl ? k : 0;
+  double *const A1c = reinterpret_cast<double *>(A1s) + ca * kKMax;
   uint32_t m0 = 0, m1 = 0, ma = 0;
+#pragma unroll 4
+  for (int r = la; r < ka; r += 16) {
+    const double v = __ldcg(A1g + (size_t)r * a.a_rs);
+    A1c[r] = v;
+    ma = max(ma, mag(v));
+  }
+  // ---- column scales: largest exponent, then the norm ----
 #pragma unroll
   for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -243,8 +308,6 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
       m0 = max(m0, mag(x[0][q][e]));
       m1 = max(m1, mag(x[1][q][e]));
     }
-#pragma unroll
-  for (int q = 0; q < kKMax / 16; ++q) ma = max(ma, mag(xa[q]));
 #pragma unroll
   for (int o = 1; o <= 2; o <<= 1) {
     m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
@@ -281,9 +344,9 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
       n0 = fmaf(f0, f0, n0);
       n1 = fmaf(f1, f1, n1);
     }
-#pragma unroll
-  for (int q = 0; q < kKMax / 16; ++q) {
-    const float f = rel(xa[q], ea);
+#pragma unroll 4
+  for (int r = la; r < ka; r += 16) {
+    const float f = rel(A1c[r], ea);
     na = fmaf(f, f, na);
   }
 #pragma unroll
@@ -300,12 +363,12 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   }
   if (la == 0) red[8 * kCols + ca] = __float_as_uint(na);
   __syncthreads();
-  // largest s with norm 2^s <= 2^60.98: norm^2 <= 3.9 * 4^h, s = 60 - h + 1022 - emax
+  // largest s with norm 2^s <= 2^60.9: norm^2 <= 3.48 * 4^h, s = 60 - h + 1022 - emax
   auto col_scale = [&](int c, int emax) {
     float n = 0.0f;
 #pragma unroll
     for (int w = 0; w < 9; ++w) n += __uint_as_float(red[w * kCols + c]);
-    const int ex = ((__float_as_int(n * (1.0f / 3.9f)) >> 23) & 0xff) - 127;   // floor(log2)
+    const int ex = ((__float_as_int(n * (1.0f / 3.48f)) >> 23) & 0xff) - 127;   // floor(log2)
     return 60 - ((ex + 2) >> 1) + 1022 - emax;
   };
   const int s0 = col_scale(g, e0), s1 = col_scale(g + 8, e1), sa = col_scale(ca, ea);
@@ -317,13 +380,8 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
       X[0][q][e] = to_fixed<true>(x[0][q][e], s0) + (long long)kBias;
       X[1][q][e] = to_fixed<true>(x[1][q][e], s1) + (long long)kBias;
     }
-  if (a.mode == 1) {
-#pragma unroll
-    for (int q = 0; q < kKMax / 16; ++q) {
-      const int r = la + 16 * q;
-      if (r < k) A1s[ca * kKMax + r] = to_fixed<true>(xa[q], sa);
-    }
-  }
+#pragma unroll 2
+  for (int r = la; r < ka; r += 16) A1s[ca * kKMax + r] = to_fixed<true>(A1c[r], sa);
 
   const int nblk = (k + ib - 1) / ib;
   const uint32_t vbase = saddr(Vd), wbase = saddr(Wd), tbase = saddr(Td);
@@ -335,71 +393,82 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
     const int wlo = r0 >> 5, whi = (Lr + 31) >> 5;      // warps that hold some of them
     const bool act = warp >= wlo && warp < whi;
     const bool two = kb > 16;                           // second half of the 32 reflectors in use
-    // ---- digits of op(T), two pairs (q, q + 1) of one row p each ----
+    // ---- digits of this warp's 32 rows of V, four pairs of reflectors at a time ----
+    double tv[2 / G][2];                                // op(T)'s entries, loaded ahead of V's digits
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int idx = tid + u * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
-      unsigned long long y[2];
+    for (int w = 0; w < 2 / G; ++w) {
+      const int idx = tid + w * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         // W2[p] = sum_q op(T)[p, q] W1[q]; op(T) = T^T reads T[q, p]
         const int row = a.transT ? q + e : p, col = a.transT ? p : q + e;
-        const double v = (row <= col && col < kb) ? __ldcg(a.T + ix(row, i + col, a.ldt)) : 0.0;
-        bad |= ((__double2hiint(v) >> 20) & 0x7ff) >= 1025;
-        y[e] = (unsigned long long)to_fixed<false>(v, 59) + kBias;
+        tv[w][e] = (row <= col && col < kb) ? __ldcg(a.T + ix(row, i + col, a.ldt)) : 0.0;
       }
-      const uint32_t off = plane_off(p, q);
-      digits(y[0], y[1], [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Td + d * kPlaneV + off) = w; });
     }
     if (act) {
-      // ---- digits of this warp's 32 rows of V ----
       const int r = 32 * warp + 2 * (lane & 15);
       const double *const Vg = a.V + ix(r, i, a.ldv);
-      const bool v16 = ((uintptr_t)Vg & 15) == 0 && (a.ldv & 1) == 0;
+      const int np = two ? 32 : 16;                    // reflectors to fill
+      const bool wholev = ((uintptr_t)Vg & 15) == 0 && (a.ldv & 1) == 0 && kb == np && 32 * warp + 32 <= Lr &&
+                          (a.mode == 0 ? 32 * warp >= i + kb : !tt || 32 * warp + 32 <= a.tt + i + 1);
+      constexpr int kStep = 8;                         // reflectors of a pass
+      int p = kStep * grp + (lane >> 4);
+      double v[4][2], n[4][2];
+      load_v(a, Vg, wholev, r, p, kb, i, Lr, tt, v);
+      if (G > 1) asm volatile("bar.sync %0, 64;" ::"r"(2 + warp) : "memory");   // the other group has read its digits
+#pragma unroll 1
+      for (; p < np; p += kStep * G) {
+        if (p + kStep * G < np) load_v(a, Vg, wholev, r, p + kStep * G, kb, i, Lr, tt, n);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (h == 1 && !two) break;
-        double v[8][2];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int p = 16 * h + 2 * u + (lane >> 4);
-          const double *vp = Vg + (size_t)p * a.ldv;
-          // rows [lo, hi) of reflector p are stored; mode 0 adds the unit row lo - 1
-          const int lo = a.mode == 0 ? r0 + p + 1 : 0;
-          const int hi = p < kb ? (tt ? min(Lr, a.tt + i + p + 1) : L) : 0;
-          v[u][0] = v[u][1] = 0.0;
-          if (v16 && r >= lo && r + 1 < hi) {
-            const double2 w = __ldcg(reinterpret_cast<const double2 *>(vp));
-            v[u][0] = w.x; v[u][1] = w.y;
-          } else {
-            if (r >= lo && r < hi) v[u][0] = __ldcg(vp);
-            if (r + 1 >= lo && r + 1 < hi) v[u][1] = __ldcg(vp + 1);
-            if (a.mode == 0 && p < kb) {
-              if (r == lo - 1) v[u][0] = 1.0;
-              if (r + 1 == lo - 1) v[u][1] = 1.0;
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int p = 16 * h + 2 * u + (lane >> 4);
-          bad |= ((__double2hiint(v[u][0]) & 0x7fffffff) >= 0x3fff0000) |
-                 ((__double2hiint(v[u][1]) & 0x7fffffff) >= 0x3fff0000);       // |v| < 1.9375
-          const unsigned long long y0 = (unsigned long long)to_fixed<false>(v[u][0], 61) + kBias;
-          const unsigned long long y1 = (unsigned long long)to_fixed<false>(v[u][1], 61) + kBias;
-          const uint32_t off = plane_off(p, 2 * (lane & 15));
+        for (int u = 0; u < 4; ++u) {
+          const unsigned long long y0 = (unsigned long long)to_fixed_max(v[u][0], 61, vmax) + kBias;
+          const unsigned long long y1 = (unsigned long long)to_fixed_max(v[u][1], 61, vmax) + kBias;
+          const uint32_t off = plane_off(p + 2 * u, 2 * (lane & 15));
           digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Vd + d * kPlaneV + off) = w; });
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { v[u][0] = n[u][0]; v[u][1] = n[u][1]; }
       }
-      __syncwarp();
+    }
+    // ---- digits of op(T), pairs (q, q + 1) of one row p ----
+#pragma unroll
+    for (int w = 0; w < 2 / G; ++w) {
+      const int idx = tid + w * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
+      const unsigned long long y0 = (unsigned long long)to_fixed_max(tv[w][0], 60, tmax) + kBias;
+      const unsigned long long y1 = (unsigned long long)to_fixed_max(tv[w][1], 60, tmax) + kBias;
+      const uint32_t off = plane_off(p, q);
+      digits(y0, y1, [&](int d, uint32_t z) { *reinterpret_cast<uint32_t *>(Td + d * kPlaneV + off) = z; });
+    }
+    if (act) {
+      if (G > 1) asm volatile("bar.sync %0, 64;" ::"r"(2 + warp) : "memory");
+      else __syncwarp();
       // ---- this warp's share of V^T C, 16 reflectors x 8 columns at a time ----
+      // a column's norm leaves its elements a few bits below the digits' range:
+      // 4 C instead of C where no element of the warp reaches 2^59
+      uint32_t far = 0;
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) far |= (uint32_t)(X[u][q][e] >> 32) - (uint32_t)(kBias >> 32) + 0x08000000u;
+      const bool up = __all_sync(0xffffffffu, far < 0x10000000u);
+      const uint32_t mul = up ? 4u : 1u;
+      const unsigned long long off = up ? 0ull - 3ull * kBias : 0ull;      // biased values: 4 (y - bias) + bias
+      if (lane == 0) shw[warp] = up ? 2u : 0u;
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         uint32_t cd[kD][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          digits((unsigned long long)X[u][q][0], (unsigned long long)X[u][q][1],
-                 [&](int d, uint32_t w) { cd[d][q] = w; });
+        for (int q = 0; q < 4; ++q) {
+          unsigned long long y[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const unsigned long long v = (unsigned long long)X[u][q][e];
+            y[e] = (unsigned long long)(uint32_t)v * mul + off + ((unsigned long long)((uint32_t)(v >> 32) * mul) << 32);
+          }
+          digits(y[0], y[1], [&](int d, uint32_t w) { cd[d][q] = w; });
+        }
 #pragma unroll 1
         for (int mt = 0; mt < (two ? 2 : 1); ++mt) {
           float acc[kD][4];
@@ -416,10 +485,10 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
                 mma(acc[d + j], av[0], av[1], av[2], av[3], cd[j][2 * kt], cd[j][2 * kt + 1]);
             }
           long long *wp = Wp + ((size_t)warp * kCols + 8 * u + 2 * t) * kLdWp + 16 * mt + g;
-          wp[0] = recon<47>(acc, 0, bad);
-          wp[kLdWp] = recon<47>(acc, 1, bad);
-          wp[8] = recon<47>(acc, 2, bad);
-          wp[kLdWp + 8] = recon<47>(acc, 3, bad);
+          wp[0] = recon<47>(acc, 0, big);
+          wp[kLdWp] = recon<47>(acc, 1, big);
+          wp[8] = recon<47>(acc, 2, big);
+          wp[kLdWp + 8] = recon<47>(acc, 3, big);
         }
       }
     }
@@ -427,16 +496,17 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
     // ---- W1 = A1 rows + the warps' shares ----
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const int q = tid & 31, c = (tid >> 5) + 8 * u;
+      const int q = gtid & 31, c = (gtid >> 5) + 8 * u;
       long long w = 0;
       if (q < kb) {
         int top = 0;
-        if (a.mode == 1) {
+        if (a.mode == 1 && c < nwl) {
           w = A1s[c * kKMax + i + q];
           top = (int)(w >> 36);
         }
         for (int ww = wlo; ww < whi; ++ww) {
-          const long long v = Wp[((size_t)ww * kCols + c) * kLdWp + q];
+          const uint32_t sh = shw[ww];
+          const long long v = (Wp[((size_t)ww * kCols + c) * kLdWp + q] + (long long)sh) >> sh;   // rounded
           w += v;
           top += (int)(v >> 36);
         }
@@ -447,110 +517,99 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
     __syncthreads();
     // ---- W2 = op(T) W1 (8 reflectors a warp), A1 -= W2, W2's digits ----
     if (warp < (two ? 4 : 2)) {
-      uint32_t wa[kD][2][4];
-#pragma unroll
-      for (int kt = 0; kt < 2; ++kt)
+      float acc[kD][4];
+      init_acc(acc);
+#pragma unroll 1
+      for (int kt = 0; kt < (two ? 2 : 1); ++kt) {
+        uint32_t wa[kD][4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const longlong2 v = *reinterpret_cast<const longlong2 *>(W1 + (g + 8 * (e & 1)) * kLdW1 + 16 * kt + 8 * (e >> 1) + 2 * t);
-          digits((unsigned long long)v.x, (unsigned long long)v.y, [&](int d, uint32_t w) { wa[d][kt][e] = w; });
+          digits((unsigned long long)v.x, (unsigned long long)v.y, [&](int d, uint32_t w) { wa[d][e] = w; });
         }
-      float acc[kD][4];
-      init_acc(acc);
 #pragma unroll
-      for (int d = 0; d < kD; ++d) {
-        uint32_t bt[4];
-        ldsm4(tbase + d * kPlaneV + plane_off(8 * warp + (lane & 7), 8 * (lane >> 3)), bt);
+        for (int d = 0; d < kD; ++d) {
+          uint32_t bt[2];
+          ldsm2(tbase + d * kPlaneV + plane_off(8 * warp + (lane & 7), 16 * kt + 8 * ((lane >> 3) & 1)), bt);
 #pragma unroll
-        for (int j = 0; j < kD - d; ++j) {
-          mma(acc[d + j], wa[j][0][0], wa[j][0][1], wa[j][0][2], wa[j][0][3], bt[0], bt[1]);
-          mma(acc[d + j], wa[j][1][0], wa[j][1][1], wa[j][1][2], wa[j][1][3], bt[2], bt[3]);
+          for (int j = 0; j < kD - d; ++j) mma(acc[d + j], wa[j][0], wa[j][1], wa[j][2], wa[j][3], bt[0], bt[1]);
         }
       }
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int c = g + 8 * u, p = 8 * warp + 2 * t;
-        const long long w0 = recon<49>(acc, 2 * u, bad), w1 = recon<49>(acc, 2 * u + 1, bad);
-        if (a.mode == 1) {
+        const long long w0 = recon<48>(acc, 2 * u, big), w1 = recon<48>(acc, 2 * u + 1, big);
+        if (a.mode == 1 && c < nwl) {
           long long *ap = A1s + c * kKMax + i + p;
-          if (p < kb) {
-            ap[0] -= w0;
-            bad |= ((uint32_t)(ap[0] >> 32) + 0x40000000u) >> 31;
-          }
-          if (p + 1 < kb) {
-            ap[1] -= w1;
-            bad |= ((uint32_t)(ap[1] >> 32) + 0x40000000u) >> 31;
-          }
+          if (p < kb) ap[0] -= w0;
+          if (p + 1 < kb) ap[1] -= w1;
         }
         const uint32_t off = plane_off(c, p);
-        digits((unsigned long long)w0 + kBias, (unsigned long long)w1 + kBias,
-               [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Wd + d * kPlaneW + off) = w; });
+        const unsigned long long y0 = (unsigned long long)w0 + kBias, y1 = (unsigned long long)w1 + kBias;
+        bad |= (int)((uint32_t)((y0 | y1) >> 32) >> 31);              // outside the digits' range
+        digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Wd + d * kPlaneW + off) = w; });
       }
     }
     __syncthreads();
     // ---- C -= V W2 on this warp's rows, 8 rows at a time ----
     if (act) {
-      uint32_t wa[kD][2][4];
-#pragma unroll
-      for (int d = 0; d < kD; ++d) {
-        ldsm4(wbase + d * kPlaneW + plane_off(lane & 15, 8 * (lane >> 4)), wa[d][0]);
-        if (two) ldsm4(wbase + d * kPlaneW + plane_off(lane & 15, 16 + 8 * (lane >> 4)), wa[d][1]);
-      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float acc[kD][4];
         init_acc(acc);
+#pragma unroll 1
+        for (int kt = 0; kt < (two ? 2 : 1); ++kt) {
+          uint32_t wa[kD][4];
 #pragma unroll
-        for (int d = 0; d < kD; ++d) {
-          uint32_t bv[4];
-          ldsm4t(vbase + d * kPlaneV + plane_off(lane, 8 * q), bv);
+          for (int d = 0; d < kD; ++d) ldsm4(wbase + d * kPlaneW + plane_off(lane & 15, 16 * kt + 8 * (lane >> 4)), wa[d]);
 #pragma unroll
-          for (int j = 0; j < kD - d; ++j) {
-            mma(acc[d + j], wa[j][0][0], wa[j][0][1], wa[j][0][2], wa[j][0][3], bv[0], bv[1]);
-            if (two) mma(acc[d + j], wa[j][1][0], wa[j][1][1], wa[j][1][2], wa[j][1][3], bv[2], bv[3]);
+          for (int d = 0; d < kD; ++d) {
+            uint32_t bv[2];
+            ldsm2t(vbase + d * kPlaneV + plane_off(16 * kt + (lane & 15), 8 * q), bv);
+#pragma unroll
+            for (int j = 0; j < kD - d; ++j) mma(acc[d + j], wa[j][0], wa[j][1], wa[j][2], wa[j][3], bv[0], bv[1]);
           }
         }
 #pragma unroll
         for (int u = 0; u < 2; ++u)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            X[u][q][e] -= recon<47>(acc, 2 * u + e, bad);
+            X[u][q][e] -= recon<47>(acc, 2 * u + e, big);
             bad |= (int)((uint32_t)(X[u][q][e] >> 32) >> 31);   // left the biased range
           }
       }
-      __syncwarp();
+      if (G == 1) __syncwarp();
     }
   }
-  if (__syncthreads_or(bad)) return false;
+  if (__syncthreads_or(bad | (int)((big & kBig) != 0) | (vmax >= 0x3fff0000u) | (tmax >= 0x400f0000u))) return false;
 
   // ---- back to FP64: the elements whose value changed ----
-  auto from_fixed = [](long long v, int s) {
-    double d = __ll2double_rn(v);
-    return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (s << 20), __double2loint(d));
-  };
+  load_c(x);
 #pragma unroll
   for (int u = 0; u < 2; ++u)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t, s = u ? s1 : s0;
       double *p = Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs;
-      if (c < nwl) {
+      double y[2];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (r + e < Lt) {
-            double *pe = p + (size_t)e * a.c_rs;
-            const long long v = X[u][q][e] - (long long)kBias;
-            if (v != to_fixed<true>(__ldcg(pe), s)) *pe = from_fixed(v, s);
-          }
-        }
+      for (int e = 0; e < 2; ++e) {
+        const long long v = X[u][q][e] - (long long)kBias;
+        y[e] = v != to_fixed<true>(x[u][q][e], s) ? from_fixed(v, s) : x[u][q][e];
+      }
+      if (whole) {
+        *reinterpret_cast<double2 *>(p) = make_double2(y[0], y[1]);
+      } else if (c < nwl) {
+        if (r < Lt) p[0] = y[0];
+        if (r + 1 < Lt) p[a.c_rs] = y[1];
       }
     }
-  if (a.mode == 1 && ca < nwl) {
-    for (int r = la; r < k; r += 16) {
-      double *pe = A1g + (size_t)r * a.a_rs;
-      const long long v = A1s[ca * kKMax + r];
-      if (v != to_fixed<true>(__ldcg(pe), sa)) *pe = from_fixed(v, sa);
-    }
+#pragma unroll 4
+  for (int r = la; r < ka; r += 16) {
+    double *pe = A1g + (size_t)r * a.a_rs;
+    const double o = __ldcg(pe);
+    const long long v = A1s[ca * kKMax + r];
+    if (v != to_fixed<true>(o, sa)) *pe = from_fixed(v, sa);
   }
   __syncthreads();
   return true;

@@ -65,8 +65,9 @@ def worst(x, y, norms):
     return float(np.max(np.linalg.norm((x - y).astype(np.float64), axis=0) / norms))
 
 
-@pytest.mark.parametrize("m,k,ib,w", [(32, 8, 8, 1), (33, 32, 32, 16), (64, 64, 16, 17), (100, 70, 24, 5),
-                                      (255, 256, 32, 31), (256, 256, 32, 48), (97, 33, 17, 16)])
+@pytest.mark.parametrize("m,k,ib,w", [(64, 33, 32, 1), (128, 32, 32, 16), (129, 64, 16, 17), (100, 70, 24, 5),
+                                      (255, 256, 32, 31), (256, 256, 32, 48), (121, 35, 17, 16),
+                                      (256, 16, 16, 40), (127, 32, 32, 3)])
 def test_tsmqr_every_edge(tq, oracle, m, k, ib, w):
     rng = np.random.default_rng(m + k)
     V, T = reflectors_ts(oracle, m, k, ib, rng)
@@ -86,7 +87,7 @@ def test_tsmqr_every_edge(tq, oracle, m, k, ib, w):
             assert worst(np.vstack([g1, g2]), np.vstack([r1, r2]), norms) <= bar
 
 
-@pytest.mark.parametrize("m,k,ib,w", [(32, 32, 32, 3), (65, 40, 16, 16), (256, 200, 32, 33), (200, 199, 31, 16),
+@pytest.mark.parametrize("m,k,ib,w", [(128, 32, 32, 3), (130, 40, 16, 16), (256, 200, 32, 33), (200, 199, 31, 16),
                                       (256, 256, 8, 16)])
 def test_unmqr_every_edge(tq, oracle, m, k, ib, w):
     rng = np.random.default_rng(3 * m + k)
