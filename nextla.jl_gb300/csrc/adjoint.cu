@@ -65,7 +65,7 @@ static size_t adj_smem(bool oz) {
 // (oz_apply.cuh, one CTA per SM) unless the blocks are too small for them.
 template <typename R>
 static bool adj_oz(int n, int ib) {
-  return std::is_same<R, double>::value && oz::covers(1, kAdjNb, n, ib);
+  return std::is_same<R, double>::value && (oz::covers(1, kAdjNb, n, ib) || blk::covers(kAdjNb, std::min(n, ib)));
 }
 
 struct AdjGeom {
@@ -179,7 +179,7 @@ __device__ void factor_one(const AdjGeom &g, R *A, R *tau, R *Tw, unsigned char 
   const int L0 = g.rows(0);
   for (int i0 = 0; i0 < n; i0 += ib) {
     const int sb = min(ib, n - i0);
-    panel_qr_cta<R>(L0 - i0, sb, A + ix(i0, i0, lda), lda, tau + i0, Tw + ix(0, i0, ib), ib, true, true, smem);
+    panel_qr_cta<R, OZ>(L0 - i0, sb, A + ix(i0, i0, lda), lda, tau + i0, Tw + ix(0, i0, ib), ib, true, true, smem);
     ApplyArgs<R> a = base_args<R>(sb);
     a.mode = 0; a.L = L0 - i0; a.k = sb;
     a.C = A + i0; a.c_cs = lda; a.ncols = n;
@@ -197,7 +197,7 @@ __device__ void factor_one(const AdjGeom &g, R *A, R *tau, R *Tw, unsigned char 
     __syncthreads();
     for (int i0 = 0; i0 < n; i0 += ib) {
       const int sb = min(ib, n - i0);
-      tsqrt_block_cta<R>(Lt, sb, A + ix(i0, i0, lda), lda, At + ix(0, i0, lda), lda, Tt + ix(0, i0, ib), ib,
+      tsqrt_block_cta<R, OZ>(Lt, sb, A + ix(i0, i0, lda), lda, At + ix(0, i0, lda), lda, Tt + ix(0, i0, ib), ib,
                          tau + (size_t)t * n + i0, true, smem);
       ApplyArgs<R> a = base_args<R>(sb);
       a.mode = 1; a.L = Lt; a.k = sb;

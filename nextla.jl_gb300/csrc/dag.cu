@@ -242,7 +242,7 @@ struct TcState {
 
 // Runs one task; false only if a TC task's tensor-core wait gave up.  TC:
 // this instantiation carries the tensor-core task (FP32 only).
-template <typename R, int NW, bool TC>
+template <typename R, int NW, bool TC, bool F64P>
 __device__ bool run_item(const DagArgs<R> &a, const DagItem &it, unsigned char *smem, TcState *tcs) {
   const DagGeom &g = a.g;
   const int nb = g.nb, ib = g.ib;
@@ -255,9 +255,9 @@ __device__ bool run_item(const DagArgs<R> &a, const DagItem &it, unsigned char *
   auto tautile = [&](int r, int c) { return a.tau + ix(c * nb, r, a.ldtau); };
   if (it.type == IT_GB) {
     R *Ab = tile(k, k) + ix(b * ib, b * ib, a.lda);
-    if constexpr (std::is_same<R, float>::value) {
+    if constexpr (F64P) {
       if (a.D) {
-        panel_qr_cta_f64(nb - b * ib, ib, Ab, a.lda, tautile(k, k) + b * ib, ttile(k, k) + ix(0, b * ib, a.ldt),
+        panel_qr_cta_f64<TC>(nb - b * ib, ib, Ab, a.lda, tautile(k, k) + b * ib, ttile(k, k) + ix(0, b * ib, a.ldt),
                          a.ldt, a.D + (size_t)(k * nb + b * ib) * ib, ib, smem);
         return true;
       }
@@ -267,13 +267,13 @@ __device__ bool run_item(const DagArgs<R> &a, const DagItem &it, unsigned char *
     return true;
   }
   if (it.type == IT_TB) {
-    if constexpr (std::is_same<R, float>::value) {
+    if constexpr (F64P) {
       if (a.D) {
         double *Dk = a.D + (size_t)(k * nb + b * ib) * ib;
         float *A1 = tile(k, k) + ix(b * ib, b * ib, a.lda), *A2 = tile(i, k) + ix(0, b * ib, a.lda);
         float *Tb = ttile(i, k) + ix(0, b * ib, a.ldt), *tb = tautile(i, k) + b * ib;
         if (ib <= 32)
-          tsqrt_block_f64x(nb, ib, Dk, ib, A1, a.lda, A2, a.lda, Tb, a.ldt, tb, smem);
+          tsqrt_block_f64x<TC>(nb, ib, Dk, ib, A1, a.lda, A2, a.lda, Tb, a.ldt, tb, smem);
         else
           tsqrt_block_cta_f64(nb, ib, Dk, ib, A1, a.lda, A2, a.lda, Tb, a.ldt, tb, smem);
         return true;
@@ -343,7 +343,9 @@ __device__ bool run_item(const DagArgs<R> &a, const DagItem &it, unsigned char *
   return true;
 }
 
-template <typename R, int NW, bool TC>
+// F64P (FP32): the panel tasks in FP64; a separate instantiation keeps their
+// registers and code away from the plain FP32 kernel.
+template <typename R, int NW, bool TC, bool F64P>
 __global__ void __launch_bounds__(TQR_THREADS, TC ? 1 : 2)
 k_tile_dag(const __grid_constant__ DagArgs<R> a)
 {
@@ -428,7 +430,7 @@ k_tile_dag(const __grid_constant__ DagArgs<R> a)
     }
     __syncthreads();
     if (s_err) break;
-    if (!run_item<R, NW, TC>(a, it, smem_raw, &tcs)) {
+    if (!run_item<R, NW, TC, F64P>(a, it, smem_raw, &tcs)) {
       // a tensor-core completion wait gave up: report, then stop this CTA
       if (tid == 0 && atomicCAS(&a.hdr->error, 0, 3) == 0) {
         a.hdr->err_item = idx;
@@ -774,32 +776,32 @@ static std::shared_ptr<Plan> get_plan(const DagGeom &g) {
   return p;
 }
 
-template <typename R, int NW, bool TC = false>
+template <typename R, int NW, bool TC = false, bool F64P = false>
 static int launch_dag(const DagArgs<R> &a, size_t sm, double flops, cudaStream_t st, bool timed = true) {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_tile_dag<R, NW, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
+  if ((e = cudaFuncSetAttribute(k_tile_dag<R, NW, TC, F64P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
       cudaSuccess)
     return (int)e;
   int dev = 0, sms = 0, per_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile_dag<R, NW, TC>, TQR_THREADS, sm)) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile_dag<R, NW, TC, F64P>, TQR_THREADS, sm)) !=
       cudaSuccess)
     return (int)e;
   if (per_sm < 1) return (int)cudaErrorInvalidConfiguration;
   const int grid = std::min(sms * per_sm, a.nitems);
   void *tok = timed ? prof_begin(st) : nullptr;
-  k_tile_dag<R, NW, TC><<<grid, TQR_THREADS, sm, st>>>(a);
+  k_tile_dag<R, NW, TC, F64P><<<grid, TQR_THREADS, sm, st>>>(a);
   if (timed) prof_end(tok, st, flops);
   count_launch();
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
 }
 
-// Double precision: whether the strip updates run on the tensor cores
-// (oz_apply.cuh), which takes one CTA per SM; panel-step strips of few rows
-// stay on the DFMA loops either way.
-static bool dag_oz(const DagGeom &g) { return oz::covers(1, g.nb, g.nb, g.ib); }
+// Double precision: whether strip updates (oz_apply.cuh) or panel steps
+// (panel_blk.cuh) use the tensor cores, which takes one CTA per SM; what the
+// two do not cover stays on the FP64 loops either way.
+static bool dag_oz(const DagGeom &g) { return oz::covers(1, g.nb, g.nb, g.ib) || blk::covers(g.nb, g.ib); }
 
 static int launch_dag_oz(const DagArgs<double> &a, size_t sm, double flops, cudaStream_t st, bool timed = true) {
   sm = std::max(sm, oz::kSmem);
@@ -873,7 +875,11 @@ static int tile_geqrf_dag(int m, int n, int nb, int ib, R *A, int lda, R *T, int
   const double mn = (double)std::max(m, n), kn = (double)std::min(m, n);
   const double flops = 2.0 * mn * kn * kn - 2.0 * kn * kn * kn / 3.0;
   if constexpr (std::is_same<R, float>::value) {
+    if (g.tc && g.f64p) return launch_dag<R, 16, true, true>(a, sm, flops, st);
     if (g.tc) return launch_dag<R, 16, true>(a, sm, flops, st);
+    if (g.f64p)
+      return g.nw == 16 ? launch_dag<R, 16, false, true>(a, sm, flops, st)
+                        : launch_dag<R, 8, false, true>(a, sm, flops, st);
   }
   if constexpr (std::is_same<R, double>::value) {
     if (dag_oz(g)) return launch_dag_oz(a, sm, flops, st);
@@ -1285,24 +1291,24 @@ int tqr_tile_dag_occupancy(int dtype_bytes, int tensor_cores, int *ctas_per_sm, 
   if (dtype_bytes == 8) {
     sm = std::max({apply_smem_elems(nb, ib, 16, true, true, true) * sizeof(double), panel_smem<double>(nb, ib, true, true),
                    tsqrt_smem<double>(nb, ib, true)});
-    if ((e = cudaFuncSetAttribute(k_tile_dag<double, 16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if ((e = cudaFuncSetAttribute(k_tile_dag<double, 16, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sm)) != cudaSuccess)
       return (int)e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<double, 16, false>, TQR_THREADS, sm);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<double, 16, false, false>, TQR_THREADS, sm);
   } else {
     sm = std::max({apply_smem_elems(nb, ib, 16, true, true, true) * sizeof(float), panel_smem<float>(nb, ib, true, true),
                    tsqrt_smem<float>(nb, ib, true)});
     if (tensor_cores) {
       sm = std::max(sm, tc::kSmem);
-      if ((e = cudaFuncSetAttribute(k_tile_dag<float, 16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if ((e = cudaFuncSetAttribute(k_tile_dag<float, 16, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sm)) != cudaSuccess)
         return (int)e;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<float, 16, true>, TQR_THREADS, sm);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<float, 16, true, false>, TQR_THREADS, sm);
     } else {
-      if ((e = cudaFuncSetAttribute(k_tile_dag<float, 16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      if ((e = cudaFuncSetAttribute(k_tile_dag<float, 16, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)sm)) != cudaSuccess)
         return (int)e;
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<float, 16, false>, TQR_THREADS, sm);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<float, 16, false, false>, TQR_THREADS, sm);
     }
   }
   if (e != cudaSuccess) return (int)e;

@@ -12,22 +12,23 @@
 
 namespace tqr {
 
-template <typename R>
+// BLK: the blocked FP64 column loop (panel_blk.cuh)
+template <typename R, bool BLK>
 __global__ void __launch_bounds__(TQR_THREADS)
 k_panel_qr(int m, int nc, R *__restrict__ A, int lda, R *__restrict__ tau,
            R *__restrict__ T, int ldt, int staged, int stage_t)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  panel_qr_cta<R>(m, nc, A, lda, tau, T, ldt, staged != 0, stage_t != 0, smem_raw);
+  panel_qr_cta<R, BLK>(m, nc, A, lda, tau, T, ldt, staged != 0, stage_t != 0, smem_raw);
 }
 
-template <typename R>
+template <typename R, bool BLK>
 __global__ void __launch_bounds__(TQR_THREADS)
 k_tsqrt_block(int m, int sb, R *__restrict__ A1, int lda1, R *__restrict__ A2, int lda2,
               R *__restrict__ T, int ldt, R *__restrict__ tau, int staged, int tt)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  tsqrt_block_cta<R>(m, sb, A1, lda1, A2, lda2, T, ldt, tau, staged != 0, smem_raw, tt);
+  tsqrt_block_cta<R, BLK>(m, sb, A1, lda1, A2, lda2, T, ldt, tau, staged != 0, smem_raw, tt);
 }
 
 template <typename E>
@@ -204,9 +205,16 @@ cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt,
   bool staged = panel_smem<R>(m, nc, true, stage_t) <= (size_t)TQR_SMEM_MAX;
   size_t sm = panel_smem<R>(m, nc, staged, stage_t);
   if (sm > (size_t)TQR_SMEM_MAX) return cudaErrorInvalidValue;
-  cudaError_t e = allow_smem(k_panel_qr<R>, sm);
+  auto kern = k_panel_qr<R, false>;
+  if constexpr (std::is_same<R, double>::value) {
+    if (staged && stage_t && blk::covers(m, nc)) {
+      kern = k_panel_qr<R, true>;
+      sm += blk::kScratch;
+    }
+  }
+  cudaError_t e = allow_smem(kern, sm);
   if (e != cudaSuccess) return e;
-  k_panel_qr<R><<<1, TQR_THREADS, sm, st>>>(m, nc, A, lda, tau, T, ldt, staged ? 1 : 0, stage_t ? 1 : 0);
+  kern<<<1, TQR_THREADS, sm, st>>>(m, nc, A, lda, tau, T, ldt, staged ? 1 : 0, stage_t ? 1 : 0);
   count_launch();
   return cudaGetLastError();
 }
@@ -224,9 +232,16 @@ cudaError_t launch_tsqrt_block(int m, int sb, R *A1, int lda1, R *A2, int lda2, 
   bool staged = tsqrt_smem<R>(mrow, sb, true) <= (size_t)TQR_SMEM_MAX;
   size_t sm = tsqrt_smem<R>(mrow, sb, staged);
   if (sm > (size_t)TQR_SMEM_MAX) return cudaErrorInvalidValue;
-  cudaError_t e = allow_smem(k_tsqrt_block<R>, sm);
+  auto kern = k_tsqrt_block<R, false>;
+  if constexpr (std::is_same<R, double>::value) {
+    if (staged && blk::covers(mrow, sb)) {
+      kern = k_tsqrt_block<R, true>;
+      sm += blk::kScratch;
+    }
+  }
+  cudaError_t e = allow_smem(kern, sm);
   if (e != cudaSuccess) return e;
-  k_tsqrt_block<R><<<1, TQR_THREADS, sm, st>>>(m, sb, A1, lda1, A2, lda2, T, ldt, tau, staged ? 1 : 0, tt);
+  kern<<<1, TQR_THREADS, sm, st>>>(m, sb, A1, lda1, A2, lda2, T, ldt, tau, staged ? 1 : 0, tt);
   count_launch();
   return cudaGetLastError();
 }

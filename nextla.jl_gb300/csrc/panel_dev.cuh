@@ -33,6 +33,7 @@
 // and T live in shared memory.
 #pragma once
 #include "common.cuh"
+#include "panel_blk.cuh"
 
 namespace tqr {
 
@@ -402,6 +403,28 @@ __device__ inline R *carve(unsigned char *&p, size_t n) {
 
 __host__ __device__ inline size_t rnd16(size_t b) { return ((b + 15) / 16) * 16; }
 
+// Copies an m-by-nc block, a thread a row, eight loads in flight (the kernels
+// that run one CTA per SM, whose panels wait on L2 otherwise).  op(value, row,
+// column) is applied on the way.
+template <typename S, typename E, typename F>
+__device__ __forceinline__ void copy_rows(const S *src, size_t lds, E *dst, size_t ldd, int m, int nc, F &&op) {
+  for (int r = threadIdx.x; r < m; r += TQR_THREADS)
+    for (int c0 = 0; c0 < nc; c0 += 8) {
+      S x[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c0 + c < nc) x[c] = __ldcg(src + r + (size_t)(c0 + c) * lds);
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        if (c0 + c < nc) dst[r + (size_t)(c0 + c) * ldd] = op(x[c], r, c0 + c);
+    }
+}
+
+// Shared memory of one CTA holding a staged panel of m rows, nc <= 32
+// columns, its T, a triangle and the blocked loop's scratch.
+static_assert(8 * ((size_t)(blk::kMaxRows + 1) * 32 + 2 * 33 * 32 + TQR_THREADS + 512) + blk::kScratch <= 206 * 1024,
+              "the kernels that run one CTA per SM have room for the blocked panel");
+
 template <typename R>
 __host__ __device__ inline size_t panel_smem(int m, int nc, bool staged, bool stage_t) {
   size_t s = rnd16(sizeof(R) * TQR_THREADS) + rnd16(sizeof(R) * nc) + rnd16(sizeof(R) * 4);
@@ -420,7 +443,10 @@ __host__ __device__ inline size_t tsqrt_smem(int m, int sb, bool staged) {
 }
 
 // geqr2 (+ T) on the m-by-nc panel A; T (nc-by-nc, ldt) may be nullptr.
-// VEC: 16-byte staging for FP32 elements (as apply_strip).
+// VEC, as in apply_strip, marks the kernels that run one CTA per SM: 16-byte
+// staging for FP32 elements; FP64 ones take the blocked column loop
+// (panel_blk.cuh) where it covers the panel, with its scratch after the
+// staged panel in the kernel's shared memory.
 template <typename R, bool VEC = false>
 __device__ void panel_qr_cta(int m, int nc, R *A, int lda, R *tau, R *T, int ldt, bool staged,
                              bool stage_t, unsigned char *smem_raw)
@@ -443,6 +469,8 @@ __device__ void panel_qr_cta(int m, int nc, R *A, int lda, R *tau, R *T, int ldt
     c.P = carve<R>(sp, (size_t)c.ldp * nc);
     if (VEC && cols16_ok(A, (size_t)lda, m)) {
       stage_cols16_f32(A, (size_t)lda, m, nc, c.P, c.ldp, false);
+    } else if constexpr (VEC && std::is_same<R, double>::value) {
+      copy_rows(A, (size_t)lda, c.P, (size_t)c.ldp, m, nc, [](double v, int, int) { return v; });
     } else {
       for (int idx = tid; idx < m * nc; idx += TQR_THREADS) {
         int r = idx % m, cc = idx / m;
@@ -460,8 +488,11 @@ __device__ void panel_qr_cta(int m, int nc, R *A, int lda, R *tau, R *T, int ldt
     // staged FP64 panel with T in shared memory: the latency-hiding column
     // loop (a one-row column, geqr2.jl:32-35, is its empty-norm case)
     if (staged && T && stage_t && nc <= 32) {
-      columns_la_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, c.d, c.part, c.scal, m, k, nc, -1, false, true,
-                        tau);
+      if (VEC && blk::covers(m, nc))
+        done = columns_blk_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, m, k, nc, -1, false, true, tau, sp);
+      if (!done)
+        columns_la_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, c.d, c.part, c.scal, m, k, nc, -1, false, true,
+                          tau);
       done = true;
     }
   }
@@ -480,6 +511,9 @@ __device__ void panel_qr_cta(int m, int nc, R *A, int lda, R *tau, R *T, int ldt
   if (staged) {
     if (VEC && cols16_ok(A, (size_t)lda, m)) {
       unstage_cols16_f32(c.P, c.ldp, m, nc, A, (size_t)lda, false);
+    } else if constexpr (VEC && std::is_same<R, double>::value) {
+      for (int r = tid; r < m; r += TQR_THREADS)
+        for (int cc = 0; cc < nc; ++cc) A[ix(r, cc, lda)] = c.P[ix(r, cc, c.ldp)];
     } else {
       for (int idx = tid; idx < m * nc; idx += TQR_THREADS) {
         int r = idx % m, cc = idx / m;
@@ -533,6 +567,10 @@ __device__ void tsqrt_block_cta(int m, int sb, R *A1, int lda1, R *A2, int lda2,
     c.P = carve<R>(sp, (size_t)c.ldp * sb);
     if (VEC && tt < 0 && cols16_ok(A2, (size_t)lda2, mrow)) {
       stage_cols16_f32(A2, (size_t)lda2, mrow, sb, c.P, c.ldp, false);
+    } else if constexpr (VEC && std::is_same<R, double>::value) {
+      // rows past the triangle may hold anything (another factor): not used
+      copy_rows(A2, (size_t)lda2, c.P, (size_t)c.ldp, mrow, sb,
+                [&](double v, int r, int cc) { return in_tri(r, cc) ? v : 0.0; });
     } else {
       for (int idx = tid; idx < mrow * sb; idx += TQR_THREADS) {
         int r = idx % mrow, cc = idx / mrow;
@@ -549,7 +587,12 @@ __device__ void tsqrt_block_cta(int m, int sb, R *A1, int lda1, R *A2, int lda2,
   bool done = false;
   if constexpr (std::is_same<R, double>::value) {
     if (staged && sb <= 32) {
-      if (tt >= 0)
+      if (VEC && blk::covers(mrow, sb))
+        done = tt >= 0 ? columns_blk_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, false, false, tau, sp)
+                       : columns_blk_f64<1>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, -1, false, false, tau, sp);
+      if (done)
+        ;
+      else if (tt >= 0)
         columns_la_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, c.d, c.part, c.scal, m, sb, sb, tt, false, false, tau);
       else
         columns_la_f64<1>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, c.d, c.part, c.scal, m, sb, sb, -1, false, false, tau);
@@ -570,6 +613,10 @@ __device__ void tsqrt_block_cta(int m, int sb, R *A1, int lda1, R *A2, int lda2,
   if (staged) {
     if (VEC && tt < 0 && cols16_ok(A2, (size_t)lda2, mrow)) {
       unstage_cols16_f32(c.P, c.ldp, mrow, sb, A2, (size_t)lda2, false);
+    } else if constexpr (VEC && std::is_same<R, double>::value) {
+      for (int r = tid; r < mrow; r += TQR_THREADS)
+        for (int cc = 0; cc < sb; ++cc)
+          if (in_tri(r, cc)) A2[ix(r, cc, lda2)] = c.P[ix(r, cc, c.ldp)];
     } else {
       for (int idx = tid; idx < mrow * sb; idx += TQR_THREADS) {
         int r = idx % mrow, cc = idx / mrow;
@@ -603,6 +650,7 @@ __host__ __device__ inline size_t tsqrt_f64_smem(int m, int sb) {
 
 // geqr2 + T of the m-by-nc FP32 panel A in FP64.  D (ldd) receives the upper
 // triangle of the first min(m, nc) rows in FP64.
+template <bool BLK>
 __device__ inline void panel_qr_cta_f64(int m, int nc, float *A, int lda, float *tau, float *T, int ldt,
                                         double *D, int ldd, unsigned char *smem_raw)
 {
@@ -618,13 +666,12 @@ __device__ inline void panel_qr_cta_f64(int m, int nc, float *A, int lda, float 
   c.ldp = odd_ld(m);
   c.P = carve<double>(sp, (size_t)c.ldp * nc);
   double *taus = carve<double>(sp, nc);
-  for (int idx = tid; idx < m * nc; idx += TQR_THREADS) {
-    const int r = idx % m, cc = idx / m;
-    c.P[ix(r, cc, c.ldp)] = (double)ldg_cg(A + ix(r, cc, lda));
-  }
+  copy_rows(A, (size_t)lda, c.P, (size_t)c.ldp, m, nc, [](float v, int, int) { return (double)v; });
   __syncthreads();
   const int k = min(m, nc);
-  if (nc <= 32) {
+  if (BLK && blk::covers(m, nc) &&
+      columns_blk_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, m, k, nc, -1, true, true, taus, sp)) {
+  } else if (nc <= 32) {
     columns_la_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, c.d, c.part, c.scal, m, k, nc, -1, true, true, taus);
   } else {
     for (int i = 0; i < k; ++i) {
@@ -721,6 +768,7 @@ __host__ __device__ inline size_t ttqrt_f64_smem(int m, int sb) {
   return tsqrt_smem<double>(m, sb, true) + rnd16(sizeof(double) * sb);
 }
 
+template <bool BLK>
 __device__ inline void ttqrt_block_cta_f64(int m, int sb, int tt, double *D1, int ldd1, float *A1, int lda1,
                                            const double *D2, int ldd2, float *A2, int lda2, float *T, int ldt,
                                            float *tau, unsigned char *smem_raw)
@@ -756,7 +804,9 @@ __device__ inline void ttqrt_block_cta_f64(int m, int sb, int tt, double *D1, in
   c.tt = tt;
   __syncthreads();
   c.rs = ldb;
-  if (sb <= 32) {
+  if (BLK && blk::covers(mrow, sb) &&
+      columns_blk_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, true, false, taus, sp)) {
+  } else if (sb <= 32) {
     columns_la_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, c.d, c.part, c.scal, m, sb, sb, tt, true, false, taus);
   } else {
     for (int i = 0; i < sb; ++i) {
@@ -810,6 +860,7 @@ __host__ __device__ inline size_t tsqrt_f64x_smem(int m, int sb) {
          rnd16(sizeof(double) * 32) + rnd16(sizeof(double) * 7 * 32);
 }
 
+template <bool BLK>
 __device__ inline void tsqrt_block_f64x(int m, int sb, double *D, int ldd, float *A1, int lda1, float *A2, int lda2,
                                         float *T, int ldt, float *tau, unsigned char *smem_raw)
 {
@@ -831,10 +882,7 @@ __device__ inline void tsqrt_block_f64x(int m, int sb, double *D, int ldd, float
       Ts[r + (size_t)cc * ldts] = (double)ldg_cg(T + ix(r, cc, ldt));   // skipped columns keep T
     }
   }
-  for (int idx = tid; idx < m * sb; idx += TQR_THREADS) {
-    const int r = idx % m, cc = idx / m;
-    P[ix(r, cc, ldp)] = (double)ldg_cg(A2 + ix(r, cc, lda2));
-  }
+  copy_rows(A2, (size_t)lda2, P, (size_t)ldp, m, sb, [](float v, int, int) { return (double)v; });
   __syncthreads();
   // Householder scalars of column c from the norm partials in part[] (warp 0)
   auto scalars = [&](int c) {
@@ -859,12 +907,16 @@ __device__ inline void tsqrt_block_f64x(int m, int sb, double *D, int ldd, float
     s = warp_sum(s);
     if (lane == 0) part[warp] = s;
   };
-  norm_partials(0);
-  __syncthreads();
-  if (warp == 0) scalars(0);
-  __syncthreads();
+  const bool done = BLK && blk::covers(m, sb) &&
+                    columns_blk_f64<1>(P, ldp, B, ldb, Ts, ldts, m, sb, sb, -1, true, false, taus, sp);
+  if (!done) {
+    norm_partials(0);
+    __syncthreads();
+    if (warp == 0) scalars(0);
+    __syncthreads();
+  }
   const int jd = tid >> 3, gd = tid & 7;
-  for (int i = 0; i < sb; ++i) {
+  for (int i = 0; i < sb && !done; ++i) {
     double *xi = P + (size_t)i * ldp;
     const double beta = scal[0], tv = scal[1], sc = scal[2];
     const bool has = scal[3] != 0.0;
@@ -965,10 +1017,8 @@ __device__ inline void tsqrt_block_f64x(int m, int sb, double *D, int ldd, float
       T[ix(r, cc, ldt)] = (float)Ts[r + (size_t)cc * ldts];
     }
   }
-  for (int idx = tid; idx < m * sb; idx += TQR_THREADS) {
-    const int r = idx % m, cc = idx / m;
-    A2[ix(r, cc, lda2)] = (float)P[ix(r, cc, ldp)];
-  }
+  for (int r = tid; r < m; r += TQR_THREADS)
+    for (int cc = 0; cc < sb; ++cc) A2[ix(r, cc, lda2)] = (float)P[ix(r, cc, ldp)];
   for (int i = tid; i < sb; i += TQR_THREADS) tau[i] = (float)taus[i];
   __syncthreads();
 }

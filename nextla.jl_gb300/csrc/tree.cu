@@ -145,7 +145,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
       const int kk = min(mi, nk), c = op.b * ib;
       if (c >= kk) return;
       const int sb = min(ib, kk - c);
-      panel_qr_cta<R>(mi - c, sb, Aik + ix(c, c, g.lda), g.lda, g.tautile(g.tau, i, k) + c,
+      panel_qr_cta<R, OZ>(mi - c, sb, Aik + ix(c, c, g.lda), g.lda, g.tautile(g.tau, i, k) + c,
                       g.ttile(g.T, i, k) + ix(0, c, g.ldt), g.ldt, true, true, smem);
       return;
     }
@@ -184,7 +184,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
       const int c = op.b * ib;
       if (c >= kt) return;
       const int sb = min(ib, kt - c);
-      tsqrt_block_cta<R>(mp, sb, Aik + ix(c, c, g.lda), g.lda, Apk + ix(0, c, g.lda), g.lda,
+      tsqrt_block_cta<R, OZ>(mp, sb, Aik + ix(c, c, g.lda), g.lda, Apk + ix(0, c, g.lda), g.lda,
                          g.ttile(g.T2, p, k) + ix(0, c, g.ldt), g.ldt, g.tautile(g.tau2, p, k) + c, true, smem,
                          op.ts ? -1 : c);
       return;
@@ -228,7 +228,7 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
 // (oz_apply.cuh; OZ below), which takes one CTA per SM.
 template <typename R>
 static bool tree_oz(int nb, int ib) {
-  return std::is_same<R, double>::value && oz::covers(1, nb, nb, ib);
+  return std::is_same<R, double>::value && (oz::covers(1, nb, nb, ib) || blk::covers(nb, ib));
 }
 
 template <typename R, bool OZ>
@@ -513,6 +513,7 @@ struct TDagArgs {
 // Panel steps of the mixed form: geqrt blocks, tsqrt merges (into a group
 // leader) and ttqrt merges (of two leaders) in FP64 with the leaders'
 // diagonal triangles kept in D (panel_dev.cuh).
+template <bool BLK>
 __device__ inline void tree_panel_f64(const TDagArgs<float> &a, const TreeOp &op, int i, unsigned char *smem) {
   const TreeGeom<float> &g = a.g;
   const int k = op.k, ib = g.ib, nk = g.cols(k), mi = g.rows(i), c = op.b * ib;
@@ -521,7 +522,7 @@ __device__ inline void tree_panel_f64(const TDagArgs<float> &a, const TreeOp &op
     const int kk = min(mi, nk);
     if (c >= kk) return;
     const int sb = min(ib, kk - c);
-    panel_qr_cta_f64(mi - c, sb, Aik + ix(c, c, g.lda), g.lda, g.tautile(g.tau, i, k) + c,
+    panel_qr_cta_f64<BLK>(mi - c, sb, Aik + ix(c, c, g.lda), g.lda, g.tautile(g.tau, i, k) + c,
                      g.ttile(g.T, i, k) + ix(0, c, g.ldt), g.ldt, a.Dtri(i, k, c), ib, smem);
     return;
   }
@@ -532,10 +533,10 @@ __device__ inline void tree_panel_f64(const TDagArgs<float> &a, const TreeOp &op
   const int sb = min(ib, kt - c);
   float *T2b = g.ttile(g.T2, p, k) + ix(0, c, g.ldt), *t2b = g.tautile(g.tau2, p, k) + c;
   if (op.ts)
-    tsqrt_block_f64x(mp, sb, a.Dtri(i, k, c), ib, Aik + ix(c, c, g.lda), g.lda, Apk + ix(0, c, g.lda), g.lda, T2b,
+    tsqrt_block_f64x<BLK>(mp, sb, a.Dtri(i, k, c), ib, Aik + ix(c, c, g.lda), g.lda, Apk + ix(0, c, g.lda), g.lda, T2b,
                      g.ldt, t2b, smem);
   else
-    ttqrt_block_cta_f64(mp, sb, c, a.Dtri(i, k, c), ib, Aik + ix(c, c, g.lda), g.lda, a.Dtri(p, k, c), ib,
+    ttqrt_block_cta_f64<BLK>(mp, sb, c, a.Dtri(i, k, c), ib, Aik + ix(c, c, g.lda), g.lda, a.Dtri(p, k, c), ib,
                         Apk + ix(0, c, g.lda), g.lda, T2b, g.ldt, t2b, smem);
 }
 
@@ -557,8 +558,9 @@ __device__ __forceinline__ unsigned long long tdag_ns() {
 
 // TC: this instantiation owns the SM's TMEM and runs the tensor-core chunk
 // tasks (FP32, one CTA per SM); the other instantiations never meet one.  OZ:
-// FP64 strips on the tensor cores.
-template <typename R, bool TC, bool OZ>
+// FP64 strips on the tensor cores.  F64P (FP32): panel steps in FP64, apart
+// from the plain FP32 kernel for the sake of its registers and code.
+template <typename R, bool TC, bool OZ, bool F64P>
 __global__ void __launch_bounds__(TQR_THREADS, TC || OZ ? 1 : 2) k_tree_dag(const __grid_constant__ TDagArgs<R> a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_it, s_err;
@@ -702,8 +704,8 @@ __global__ void __launch_bounds__(TQR_THREADS, TC || OZ ? 1 : 2) k_tree_dag(cons
         } else {
           ok = false;   // never scheduled without the tensor-core instantiation
         }
-      } else if (a.D && (op.type == OP_GE_PANEL || op.type == OP_PR_PANEL)) {
-        tree_panel_f64(a, op, it.i, smem);
+      } else if (F64P && (op.type == OP_GE_PANEL || op.type == OP_PR_PANEL)) {
+        if constexpr (F64P) tree_panel_f64<TC>(a, op, it.i, smem);
       } else {
         tree_task<R, OZ>(a.g, op, it.i, it.y, smem);
       }
@@ -1102,21 +1104,21 @@ static size_t tree_work_bytes(TreeShape sh) {
   return b;
 }
 
-template <typename R, bool TC, bool OZ = false>
+template <typename R, bool TC, bool OZ = false, bool F64P = false>
 static cudaError_t tree_dag_launch(const TDagArgs<R> &a, size_t sm, cudaStream_t st) {
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_tree_dag<R, TC, OZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
+  if ((e = cudaFuncSetAttribute(k_tree_dag<R, TC, OZ, F64P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
       cudaSuccess)
     return e;
   int dev = 0, sms = 0, per_sm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tree_dag<R, TC, OZ>, TQR_THREADS, sm)) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tree_dag<R, TC, OZ, F64P>, TQR_THREADS, sm)) !=
       cudaSuccess)
     return e;
   if (per_sm < 1) return cudaErrorInvalidConfiguration;
   const int grid = std::min(sms * per_sm, a.nitems);
-  k_tree_dag<R, TC, OZ><<<grid, TQR_THREADS, sm, st>>>(a);
+  k_tree_dag<R, TC, OZ, F64P><<<grid, TQR_THREADS, sm, st>>>(a);
   count_launch();
   return cudaGetLastError();
 }
@@ -1190,13 +1192,20 @@ static int tree_geqrf_dag_impl(int m, int n, int nb, int ib, R *A, int lda, R *T
     sm = std::max({sm, panel_f64_smem(nb, ib), tsqrt_f64x_smem(nb, ib), ttqrt_f64_smem(nb, ib)});
   if constexpr (std::is_same<R, float>::value) {
     if (sh.tc) {
-      e = tree_dag_launch<R, true>(a, std::max({sm, tc::kSmem, tc::wy::kSmem}), st);
+      const size_t smt = std::max({sm, tc::kSmem, tc::wy::kSmem});
+      e = sh.f64p ? tree_dag_launch<R, true, false, true>(a, smt, st) : tree_dag_launch<R, true>(a, smt, st);
       return e == cudaSuccess ? 0 : (int)e;
     }
   }
   if constexpr (std::is_same<R, double>::value) {
     if (tree_oz<R>(nb, ib)) {
       e = tree_dag_launch<R, false, true>(a, std::max(sm, oz::kSmem), st);
+      return e == cudaSuccess ? 0 : (int)e;
+    }
+  }
+  if constexpr (std::is_same<R, float>::value) {
+    if (sh.f64p) {
+      e = tree_dag_launch<R, false, false, true>(a, sm, st);
       return e == cudaSuccess ? 0 : (int)e;
     }
   }
