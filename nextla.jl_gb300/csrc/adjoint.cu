@@ -103,7 +103,7 @@ struct AdjArgs {
 template <typename R, bool OZ>
 __device__ void apply_cols(ApplyArgs<R> a, int c0, unsigned char *smem) {
   for (int c = c0; c < a.ncols; c += AdjNW<R>::value) {
-    apply_strip<R, AdjNW<R>::value, OZ>(a, c, smem);
+    a.reuse = apply_strip<R, AdjNW<R>::value, OZ>(a, c, smem);
     __syncthreads();
   }
 }

@@ -20,7 +20,7 @@ __global__ void __launch_bounds__(TQR_THREADS, 1)
 k_apply_oz(const ApplyArgs<double> a)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  apply_strip<double, oz::kCols, true>(a, blockIdx.x * oz::kCols, smem_raw);
+  apply_strip<double, oz::kCols, 2>(a, blockIdx.x * oz::kCols, smem_raw);
 }
 
 static cudaError_t launch_oz(ApplyArgs<double> a, cudaStream_t st) {

@@ -56,6 +56,8 @@ struct ApplyArgs {
                  // [0, tt + q] only (ttmqr!/parfb! with a triangular part,
                  // src/ttmqr.jl:60-90, src/pamm.jl:104-127); rows below are
                  // never read and region rows past tt + q are not touched
+  int reuse = 0; // the previous call, with this V and T and one block, returned
+                 // true: their digits are still in shared memory
 };
 
 }  // namespace tqr
@@ -144,17 +146,22 @@ __device__ __forceinline__ void phase1_blocked_f32(const float *Vp, int ldvp, co
 // kernel runs one CTA per SM, with registers to spare.  FP32 elements then
 // take 16-byte staging of C and V; FP64 ones run on the tensor cores
 // (oz_apply.cuh, the kernel has oz::kSmem bytes of dynamic shared memory)
-// wherever the shape is covered.
-template <typename R, int NW, bool VEC = false>
-__device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_raw)
+// wherever the shape is covered; VEC = 2 also takes 257 to 512 rows.  Returns
+// true if the next strip of the same V and T may set reuse.
+template <typename R, int NW, int VEC = 0>
+__device__ bool apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_raw)
 {
   const int tid = threadIdx.x;
   const int nwl = min(NW, a.ncols - c0);
-  if (nwl <= 0) return;
-  if constexpr (VEC && std::is_same<R, double>::value && NW <= oz::kCols) {
-    if (oz::covers(a.mode, a.L, a.k, a.ib) && 
-        oz::strip<1>(a, c0, nwl, smem_raw, reinterpret_cast<long long *>(smem_raw + oz::kOffA1)))
-      return;
+  if (nwl <= 0) return false;
+  if constexpr (VEC != 0 && std::is_same<R, double>::value && NW <= oz::kCols) {
+    if (oz::covers(a.mode, a.L, a.k, a.ib)) {
+      if (a.L <= 256) {
+        if (oz::strip<1>(a, c0, nwl, smem_raw, a.reuse != 0)) return a.k <= a.ib;
+      } else if constexpr (VEC == 2) {
+        if (oz::strip<2>(a, c0, nwl, smem_raw, false)) return false;
+      }
+    }
   }
   const int L = a.L, ib = a.ib;
   const int ldw = ib;
@@ -175,7 +182,7 @@ __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_r
   const bool cjc = a.conj_c != 0;
   if (a.stage_c) {
     Cp = Cs; crs = 1; ccs = ldcs;
-    if (VEC && a.c_rs == 1 && cols16_ok(Cg, (size_t)a.c_cs, L)) {
+    if (VEC != 0 && a.c_rs == 1 && cols16_ok(Cg, (size_t)a.c_cs, L)) {
       stage_cols16_f32(Cg, (size_t)a.c_cs, L, nwl, Cs, ldcs, cjc);
     } else if (a.c_rs == 1) {
       for (int idx = tid; idx < L * nwl; idx += TQR_THREADS) {
@@ -205,7 +212,7 @@ __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_r
     // V block: element (rr, p) = reflector i+p at region row r0+rr
     const R *Vp;
     int ldvp;
-    if (VEC && a.stage_v && a.mode == 1 && !ttb && cols16_ok(a.V + ix(0, i, a.ldv), (size_t)a.ldv, Lr)) {
+    if (VEC != 0 && a.stage_v && a.mode == 1 && !ttb && cols16_ok(a.V + ix(0, i, a.ldv), (size_t)a.ldv, Lr)) {
       // every row of every reflector is stored: a plain column-block copy
       stage_cols16_f32(a.V + ix(0, i, a.ldv), (size_t)a.ldv, Lr, kb, Vs, ldvs, false);
       Vp = Vs; ldvp = ldvs;
@@ -256,7 +263,7 @@ __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_r
       Ws[p + c * ldw] = w;
     };
     bool blocked = false;
-    if constexpr (VEC && std::is_same<R, float>::value && NW == 16) {
+    if constexpr (VEC != 0 && std::is_same<R, float>::value && NW == 16) {
       // tensor-core instantiation: 16 x 32 W of a full 256-row block through
       // 4 x 4 register blocks; the eight row-group sums are added in order
       if (a.mode == 1 && !ttb && kb == 32 && nwl == 16 && Lr == 256 && a.stage_v && a.stage_c && !cjg) {
@@ -417,7 +424,7 @@ __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_r
     __syncthreads();
   }
   if (a.stage_c) {
-    if (VEC && a.c_rs == 1 && cols16_ok(Cg, (size_t)a.c_cs, L)) {
+    if (VEC != 0 && a.c_rs == 1 && cols16_ok(Cg, (size_t)a.c_cs, L)) {
       unstage_cols16_f32(Cs, ldcs, L, nwl, Cg, (size_t)a.c_cs, cjc);
     } else if (a.c_rs == 1) {
       for (int idx = tid; idx < L * nwl; idx += TQR_THREADS) {
@@ -431,6 +438,7 @@ __device__ void apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_r
       }
     }
   }
+  return false;
 }
 
 }  // namespace tqr

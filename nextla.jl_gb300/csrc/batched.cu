@@ -66,18 +66,22 @@ __host__ __device__ inline bool problem_ok(const BatchProblem &p) {
          p.ib >= 1 && p.ib <= kBatchMaxIb && (p.nw == 8 || p.nw == 16) && p.a_off >= 0 && p.b_off >= 0;
 }
 
-template <typename R, int NW>
-__device__ void update_columns(ApplyArgs<R> a, R *C, int ldc, int ncols, unsigned char *smem) {
+// OZ (FP64): panel and updates on the tensor cores (panel_blk.cuh,
+// oz_apply.cuh), one CTA per SM.
+template <typename R, int NW, bool OZ>
+__device__ bool update_columns(ApplyArgs<R> a, R *C, int ldc, int ncols, unsigned char *smem, bool reuse) {
   a.C = C; a.c_cs = ldc; a.ncols = ncols; a.nw = NW;
+  a.reuse = reuse;
   for (int c0 = 0; c0 < ncols; c0 += NW) {
-    apply_strip<R, NW>(a, c0, smem);
+    a.reuse = apply_strip<R, NW, OZ ? 2 : 0>(a, c0, smem);
     __syncthreads();
   }
+  return a.reuse != 0;
 }
 
 // One problem, one CTA: blocked Householder QR of A with the reflectors also
 // applied to B, then R X = (Q^T B)[0:n] in place of B's first n rows.
-template <typename R>
+template <typename R, bool OZ>
 __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R *tauscr, unsigned char *smem)
 {
   const int m = p.m, n = p.n, k = p.k, ib = p.ib;
@@ -87,8 +91,8 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
   for (int i = 0; i < n; i += ib) {
     const int sb = min(ib, n - i);
     const int L = m - i;
-    const bool pst = panel_smem<R>(L, sb, true, true) <= kBatchSmem;
-    panel_qr_cta<R>(L, sb, A + ix(i, i, lda), lda, tauscr + i, Tscr, ib, pst, true, smem);
+    const bool pst = OZ || panel_smem<R>(L, sb, true, true) <= kBatchSmem;
+    panel_qr_cta<R, OZ>(L, sb, A + ix(i, i, lda), lda, tauscr + i, Tscr, ib, pst, true, smem);
     ApplyArgs<R> a;
     a.mode = 0; a.L = L; a.k = sb; a.ib = sb; a.fwd = 1; a.transT = 1;
     a.c_rs = 1; a.A1 = nullptr; a.a_rs = 1; a.a_cs = 1;
@@ -96,16 +100,18 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
     a.T = Tscr; a.ldt = ib;
     a.stage_t = 1;
     const int nw = p.nw;
-    const bool full = apply_smem_elems(L, sb, nw, true, true, true) * sizeof(R) <= kBatchSmem;
+    constexpr size_t cap = OZ ? oz::kSmem : kBatchSmem;
+    const bool full = apply_smem_elems(L, sb, nw, true, true, true) * sizeof(R) <= cap;
     a.stage_v = full;
-    a.stage_c = full || apply_smem_elems(L, sb, nw, true, false, true) * sizeof(R) <= kBatchSmem;
+    a.stage_c = full || apply_smem_elems(L, sb, nw, true, false, true) * sizeof(R) <= cap;
     const int nt = n - i - sb;
+    bool reuse = false;
     if (nw == 16) {
-      if (nt > 0) update_columns<R, 16>(a, A + ix(i, i + sb, lda), lda, nt, smem);
-      if (k > 0) update_columns<R, 16>(a, B + i, ldb, k, smem);
+      if (nt > 0) reuse = update_columns<R, 16, OZ>(a, A + ix(i, i + sb, lda), lda, nt, smem, false);
+      if (k > 0) update_columns<R, 16, OZ>(a, B + i, ldb, k, smem, reuse);
     } else {
-      if (nt > 0) update_columns<R, 8>(a, A + ix(i, i + sb, lda), lda, nt, smem);
-      if (k > 0) update_columns<R, 8>(a, B + i, ldb, k, smem);
+      if (nt > 0) reuse = update_columns<R, 8, OZ>(a, A + ix(i, i + sb, lda), lda, nt, smem, false);
+      if (k > 0) update_columns<R, 8, OZ>(a, B + i, ldb, k, smem, reuse);
     }
   }
   if (k == 0) return;
@@ -134,8 +140,13 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
   __syncthreads();
 }
 
+template <typename R> constexpr bool kBatchOz = std::is_same<R, double>::value;
+template <typename R> constexpr size_t kBatchDynSmem = kBatchOz<R> ? oz::kSmem : kBatchSmem;
+static_assert(sizeof(double) * ((size_t)513 * 32 + 33 * 32 + TQR_THREADS + 64) + blk::kScratch <= oz::kSmem,
+              "a staged 512-row panel with the blocked loop's scratch");
+
 template <typename R>
-__global__ void __launch_bounds__(TQR_THREADS, 2)
+__global__ void __launch_bounds__(TQR_THREADS, kBatchOz<R> ? 1 : 2)
 k_batched_gels(int nprob, const BatchProblem *__restrict__ probs, const int *__restrict__ order, R *A, R *B,
                BatchHeader *hdr, R *scratch)
 {
@@ -159,7 +170,7 @@ k_batched_gels(int nprob, const BatchProblem *__restrict__ probs, const int *__r
       if (threadIdx.x == 0) { atomicAdd(&hdr->bad, 1); atomicMin(&hdr->first_bad, id); }
       continue;
     }
-    solve_one<R>(p, A, B, Tscr, tauscr, smem_raw);
+    solve_one<R, kBatchOz<R>>(p, A, B, Tscr, tauscr, smem_raw);
   }
 }
 
@@ -197,10 +208,10 @@ static LaunchCfg launch_cfg() {
   int sms = 0, per_sm = 0;
   if ((c.err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return c;
   if ((c.err = cudaFuncSetAttribute(k_batched_gels<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kBatchSmem)) != cudaSuccess)
+                                    (int)kBatchDynSmem<R>)) != cudaSuccess)
     return c;
   if ((c.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_gels<R>, TQR_THREADS,
-                                                             kBatchSmem)) != cudaSuccess)
+                                                             kBatchDynSmem<R>)) != cudaSuccess)
     return c;
   g.grid = sms * std::max(per_sm, 1);
   return g;
@@ -229,7 +240,7 @@ static int batched_launch(int nprob, const void *probs, const int *order, R *A, 
   count_launch();
   if (nprob > 0) {
     const int grid = std::min(c.grid, nprob);
-    k_batched_gels<R><<<grid, TQR_THREADS, kBatchSmem, st>>>(nprob, (const BatchProblem *)probs, order, A, B,
+    k_batched_gels<R><<<grid, TQR_THREADS, kBatchDynSmem<R>, st>>>(nprob, (const BatchProblem *)probs, order, A, B,
                                                              hdr, scratch);
     count_launch();
   }

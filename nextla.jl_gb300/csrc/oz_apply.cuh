@@ -51,24 +51,22 @@ template <typename R> struct ApplyArgs;
 
 namespace oz {
 
-constexpr int kCols = 16;              // strip columns of a group of eight warps
-constexpr int kRowsMax = 256;          // region rows: 32 per warp
+constexpr int kCols = 16;              // strip columns
+constexpr int kRowsMax = 512;          // region rows: 32 per warp, or two such chunks 256 apart
 constexpr int kIbMax = 32;
 constexpr int kKMax = 256;             // reflectors of a mode 1 apply (A1 rows kept until the end)
 constexpr uint32_t kPlaneV = 32 * 64;  // one digit plane of 32 rows of V: 32 reflectors x 32 rows
 constexpr uint32_t kWarpV = kD * kPlaneV;
 constexpr uint32_t kPlaneW = 16 * 64;
 constexpr int kLdWp = 36, kLdW1 = 40;
-// shared memory: V digits | T digits, then per group: W digits | partial W |
-// W | reductions, then (one group) A1
+// shared memory: V digits | T digits | W digits | W | partial W | reductions | A1
 constexpr size_t kOffT = 8 * (size_t)kWarpV;
-constexpr size_t kOffG = kOffT + kD * (size_t)kPlaneV;
-constexpr size_t kGrpW1 = kD * (size_t)kPlaneW;
-constexpr size_t kGrpWp = kGrpW1 + sizeof(long long) * kCols * kLdW1;
-constexpr size_t kGrpRed = kGrpWp + sizeof(long long) * 8 * kCols * kLdWp;
-constexpr size_t kGrpSh = kGrpRed + sizeof(uint32_t) * kCols * 9;
-constexpr size_t kGrp = kGrpSh + sizeof(uint32_t) * 16;
-constexpr size_t kOffA1 = kOffG + kGrp;
+constexpr size_t kOffW = kOffT + kD * (size_t)kPlaneV;
+constexpr size_t kOffW1 = kOffW + kD * (size_t)kPlaneW;
+constexpr size_t kOffWp = kOffW1 + sizeof(long long) * kCols * kLdW1;
+constexpr size_t kOffRed = kOffWp + sizeof(long long) * 8 * kCols * kLdWp;
+constexpr size_t kOffSh = kOffRed + sizeof(uint32_t) * kCols * 9;
+constexpr size_t kOffA1 = kOffSh + sizeof(uint32_t) * 16;
 constexpr size_t kSmem = kOffA1 + sizeof(long long) * kCols * kKMax;
 static_assert(kSmem <= TQR_SMEM_MAX, "one CTA's shared memory");
 
@@ -116,25 +114,20 @@ __device__ __forceinline__ void load_v(const ApplyArgs<double> &a, const double 
   }
 }
 
-// Applies to the strip of columns [c0, c0 + nwl), nwl <= 16 G, with G groups
-// of 256 threads, 16 columns each, sharing V's and T's digits.  a1buf: 16 G x
-// kKMax values (mode 1).  False: the strip needs the DFMA path; nothing has
-// been written.  All threads get the same answer.
-template <int G>
-__device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem,
-                                   long long *a1buf) {
-  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int grp = G == 1 ? 0 : tid >> 8, gtid = tid & 255, warp = gtid >> 5;
+// Applies to the strip of columns [c0, c0 + nwl), nwl <= 16, over at most 256
+// J rows.  reuse: V and T are those of the strip just done (true returned, one
+// block, J = 1), their digits still in place.  False: the strip needs the DFMA
+// path; nothing has been written.  All threads get the same answer.
+template <int J>
+__device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem, bool reuse) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int L = a.L, ib = a.ib, k = a.k;
-  unsigned char *const Vd = smem + (size_t)warp * kWarpV, *const Td = smem + kOffT;
-  unsigned char *const gs = smem + kOffG + grp * kGrp, *const Wd = gs;
-  long long *const W1 = reinterpret_cast<long long *>(gs + kGrpW1);
-  long long *const Wp = reinterpret_cast<long long *>(gs + kGrpWp);
-  uint32_t *const red = reinterpret_cast<uint32_t *>(gs + kGrpRed);   // [warp 0..7, A1][column]
-  uint32_t *const shw = reinterpret_cast<uint32_t *>(gs + kGrpSh);    // per warp: V^T C's share is scaled by 2^shw
-  long long *const A1s = a1buf + (size_t)grp * kCols * kKMax;
-  c0 += kCols * grp;
-  nwl = min(kCols, nwl - kCols * grp);
+  unsigned char *const Vd = smem + (size_t)warp * kWarpV, *const Td = smem + kOffT, *const Wd = smem + kOffW;
+  long long *const W1 = reinterpret_cast<long long *>(smem + kOffW1);
+  long long *const Wp = reinterpret_cast<long long *>(smem + kOffWp);
+  uint32_t *const red = reinterpret_cast<uint32_t *>(smem + kOffRed);   // [warp 0..7, A1][column]
+  uint32_t *const shw = reinterpret_cast<uint32_t *>(smem + kOffSh);    // per warp: V^T C's share is scaled by 2^shw
+  long long *const A1s = reinterpret_cast<long long *>(smem + kOffA1);
   const bool tt = a.mode == 1 && a.tt >= 0;
   const int Lt = tt ? min(L, a.tt + k) : L;            // rows any reflector touches
   int bad = 0;
@@ -143,17 +136,16 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   // ---- the strip, and A1's rows, from global memory ----
   double *const Cg = a.C + (size_t)c0 * a.c_cs;
   const bool vec = a.c_rs == 1 && ((uintptr_t)Cg & 15) == 0 && (a.c_cs & 1) == 0;
-  // this lane's elements of the strip: 16-byte loads, all in flight, where the
+  // this lane's elements of a chunk: 16-byte loads, all in flight, where the
   // warp's 32 x 16 block is whole and aligned
-  const bool whole = vec && nwl == kCols && 32 * warp + 32 <= Lt;
-  auto load_c = [&](double (&x)[2][4][2]) {
-    if (whole) {
+  auto load_c = [&](int ch, double (&x)[2][4][2]) {
+    const int r0 = 256 * ch + 32 * warp;
+    if (vec && nwl == kCols && r0 + 32 <= Lt) {
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const double2 v = __ldcg(reinterpret_cast<const double2 *>(Cg + 32 * warp + 8 * q + 2 * t +
-                                                                     (size_t)(g + 8 * u) * a.c_cs));
+          const double2 v = __ldcg(reinterpret_cast<const double2 *>(Cg + r0 + 8 * q + 2 * t + (size_t)(g + 8 * u) * a.c_cs));
           x[u][q][0] = v.x; x[u][q][1] = v.y;
         }
     } else {
@@ -163,18 +155,19 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         for (int q = 0; q < 4; ++q)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t + e;
+            const int c = g + 8 * u, r = r0 + 8 * q + 2 * t + e;
             x[u][q][e] = (c < nwl && r < Lt) ? __ldcg(Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs) : 0.0;
           }
     }
   };
-  double x[2][4][2];
-  load_c(x);
+  double x[J][2][4][2];
+#pragma unroll
+  for (int ch = 0; ch < J; ++ch) load_c(ch, x[ch]);
   // high word of |v|, nonzero for every nonzero v
   auto mag = [](double v) {
     return ((uint32_t)__double2hiint(v) & 0x7fffffffu) | (__double2loint(v) != 0 ? 1u : 0u);
   };
-  const int ca = gtid >> 4, la = gtid & 15;            // A1: 16 threads a column
+  const int ca = tid >> 4, la = tid & 15;              // A1: 16 threads a column
   double *const A1g = a.mode == 1 ? a.A1 + (size_t)(c0 + ca) * a.a_cs : nullptr;
   const int ka = a.mode == 1 && ca < nwl ? k : 0;
   double *const A1c = reinterpret_cast<double *>(A1s) + ca * kKMax;
@@ -187,12 +180,14 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   }
   // ---- column scales: largest exponent, then the norm ----
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int ch = 0; ch < J; ++ch)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      m0 = max(m0, mag(x[0][q][e]));
-      m1 = max(m1, mag(x[1][q][e]));
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        m0 = max(m0, mag(x[ch][0][q][e]));
+        m1 = max(m1, mag(x[ch][1][q][e]));
+      }
 #pragma unroll
   for (int o = 1; o <= 2; o <<= 1) {
     m0 = max(m0, __shfl_xor_sync(0xffffffffu, m0, o));
@@ -222,13 +217,15 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   };
   float n0 = 0.0f, n1 = 0.0f, na = 0.0f;
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int ch = 0; ch < J; ++ch)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float f0 = rel(x[0][q][e], e0), f1 = rel(x[1][q][e], e1);
-      n0 = fmaf(f0, f0, n0);
-      n1 = fmaf(f1, f1, n1);
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const float f0 = rel(x[ch][0][q][e], e0), f1 = rel(x[ch][1][q][e], e1);
+        n0 = fmaf(f0, f0, n0);
+        n1 = fmaf(f1, f1, n1);
+      }
 #pragma unroll 4
   for (int r = la; r < ka; r += 16) {
     const float f = rel(A1c[r], ea);
@@ -257,14 +254,17 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
     return 60 - ((ex + 2) >> 1) + 1022 - emax;
   };
   const int s0 = col_scale(g, e0), s1 = col_scale(g + 8, e1), sa = col_scale(ca, ea);
-  long long X[2][4][2];                                // biased by kBias
+  long long X[J][2][4][2];                             // biased by kBias
+  uint32_t changed = 0;                                // J = 1: elements some block moved
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int ch = 0; ch < J; ++ch)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      X[0][q][e] = to_fixed<true>(x[0][q][e], s0) + (long long)kBias;
-      X[1][q][e] = to_fixed<true>(x[1][q][e], s1) + (long long)kBias;
-    }
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        X[ch][0][q][e] = to_fixed<true>(x[ch][0][q][e], s0) + (long long)kBias;
+        X[ch][1][q][e] = to_fixed<true>(x[ch][1][q][e], s1) + (long long)kBias;
+      }
 #pragma unroll 2
   for (int r = la; r < ka; r += 16) A1s[ca * kKMax + r] = to_fixed<true>(A1c[r], sa);
 
@@ -275,35 +275,34 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
     const int kb = min(ib, k - i);
     const int r0 = a.mode == 0 ? i : 0;
     const int Lr = tt ? min(L, a.tt + i + kb) : L;      // rows this block touches: [r0, Lr)
-    const int wlo = r0 >> 5, whi = (Lr + 31) >> 5;      // warps that hold some of them
-    const bool act = warp >= wlo && warp < whi;
     const bool two = kb > 16;                           // second half of the 32 reflectors in use
-    // ---- digits of this warp's 32 rows of V, four pairs of reflectors at a time ----
-    double tv[2 / G][2];                                // op(T)'s entries, loaded ahead of V's digits
+    // whether this warp's chunk ch holds rows the block touches
+    auto active = [&](int ch, int w) { return 256 * ch + 32 * w < Lr && 256 * ch + 32 * w + 32 > r0; };
+    double tv[2][2];                                    // op(T)'s entries, loaded ahead of V's digits
 #pragma unroll
-    for (int w = 0; w < 2 / G; ++w) {
+    for (int w = 0; w < 2; ++w) {
       const int idx = tid + w * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         // W2[p] = sum_q op(T)[p, q] W1[q]; op(T) = T^T reads T[q, p]
         const int row = a.transT ? q + e : p, col = a.transT ? p : q + e;
-        tv[w][e] = (row <= col && col < kb) ? __ldcg(a.T + ix(row, i + col, a.ldt)) : 0.0;
+        tv[w][e] = (!reuse && row <= col && col < kb) ? __ldcg(a.T + ix(row, i + col, a.ldt)) : 0.0;
       }
     }
-    if (act) {
-      const int r = 32 * warp + 2 * (lane & 15);
+    // digits of 32 rows of V (chunk ch), four pairs of reflectors at a time
+    auto v_chunk = [&](int ch) {
+      const int rw = 256 * ch + 32 * warp, r = rw + 2 * (lane & 15);
       const double *const Vg = a.V + ix(r, i, a.ldv);
       const int np = two ? 32 : 16;                    // reflectors to fill
-      const bool wholev = ((uintptr_t)Vg & 15) == 0 && (a.ldv & 1) == 0 && kb == np && 32 * warp + 32 <= Lr &&
-                          (a.mode == 0 ? 32 * warp >= i + kb : !tt || 32 * warp + 32 <= a.tt + i + 1);
+      const bool wholev = ((uintptr_t)Vg & 15) == 0 && (a.ldv & 1) == 0 && kb == np && rw + 32 <= Lr &&
+                          (a.mode == 0 ? rw >= i + kb : !tt || rw + 32 <= a.tt + i + 1);
       constexpr int kStep = 8;                         // reflectors of a pass
-      int p = kStep * grp + (lane >> 4);
+      int p = lane >> 4;
       double v[4][2], n[4][2];
       load_v(a, Vg, wholev, r, p, kb, i, Lr, tt, v);
-      if (G > 1) asm volatile("bar.sync %0, 64;" ::"r"(2 + warp) : "memory");   // the other group has read its digits
 #pragma unroll 1
-      for (; p < np; p += kStep * G) {
-        if (p + kStep * G < np) load_v(a, Vg, wholev, r, p + kStep * G, kb, i, Lr, tt, n);
+      for (; p < np; p += kStep) {
+        if (p + kStep < np) load_v(a, Vg, wholev, r, p + kStep, kb, i, Lr, tt, n);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const unsigned long long y0 = (unsigned long long)to_fixed_max(v[u][0], 61, vmax) + kBias;
@@ -314,33 +313,41 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
 #pragma unroll
         for (int u = 0; u < 4; ++u) { v[u][0] = n[u][0]; v[u][1] = n[u][1]; }
       }
-    }
+      __syncwarp();
+    };
+    if (!reuse && active(0, warp)) v_chunk(0);
     // ---- digits of op(T), pairs (q, q + 1) of one row p ----
+    if (!reuse) {
 #pragma unroll
-    for (int w = 0; w < 2 / G; ++w) {
-      const int idx = tid + w * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
-      const unsigned long long y0 = (unsigned long long)to_fixed_max(tv[w][0], 60, tmax) + kBias;
-      const unsigned long long y1 = (unsigned long long)to_fixed_max(tv[w][1], 60, tmax) + kBias;
-      const uint32_t off = plane_off(p, q);
-      digits(y0, y1, [&](int d, uint32_t z) { *reinterpret_cast<uint32_t *>(Td + d * kPlaneV + off) = z; });
+      for (int w = 0; w < 2; ++w) {
+        const int idx = tid + w * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
+        const unsigned long long y0 = (unsigned long long)to_fixed_max(tv[w][0], 60, tmax) + kBias;
+        const unsigned long long y1 = (unsigned long long)to_fixed_max(tv[w][1], 60, tmax) + kBias;
+        const uint32_t off = plane_off(p, q);
+        digits(y0, y1, [&](int d, uint32_t z) { *reinterpret_cast<uint32_t *>(Td + d * kPlaneV + off) = z; });
+      }
     }
-    if (act) {
-      if (G > 1) asm volatile("bar.sync %0, 64;" ::"r"(2 + warp) : "memory");
-      else __syncwarp();
-      // ---- this warp's share of V^T C, 16 reflectors x 8 columns at a time ----
-      // a column's norm leaves its elements a few bits below the digits' range:
-      // 4 C instead of C where no element of the warp reaches 2^59
-      uint32_t far = 0;
+    // ---- this warp's share of V^T C, 16 reflectors x 8 columns at a time ----
+    // a column's norm leaves its elements a few bits below the digits' range:
+    // 4 C instead of C where no element of the warp reaches 2^59
+    uint32_t far = 0;
+#pragma unroll
+    for (int ch = 0; ch < J; ++ch)
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) far |= (uint32_t)(X[u][q][e] >> 32) - (uint32_t)(kBias >> 32) + 0x08000000u;
-      const bool up = __all_sync(0xffffffffu, far < 0x10000000u);
-      const uint32_t mul = up ? 4u : 1u;
-      const unsigned long long off = up ? 0ull - 3ull * kBias : 0ull;      // biased values: 4 (y - bias) + bias
-      if (lane == 0) shw[warp] = up ? 2u : 0u;
+          for (int e = 0; e < 2; ++e) far |= (uint32_t)(X[ch][u][q][e] >> 32) - (uint32_t)(kBias >> 32) + 0x08000000u;
+    const bool up = __all_sync(0xffffffffu, far < 0x10000000u);
+    const uint32_t mul = up ? 4u : 1u;
+    const unsigned long long off4 = up ? 0ull - 3ull * kBias : 0ull;       // biased values: 4 (y - bias) + bias
+    if (lane == 0) shw[warp] = up ? 2u : 0u;
+    bool any = false;                                   // this warp's share has been started
+#pragma unroll
+    for (int ch = 0; ch < J; ++ch) {
+      if (!active(ch, warp)) continue;
+      if (ch > 0) v_chunk(ch);
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         uint32_t cd[kD][4];
@@ -349,8 +356,8 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
           unsigned long long y[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const unsigned long long v = (unsigned long long)X[u][q][e];
-            y[e] = (unsigned long long)(uint32_t)v * mul + off + ((unsigned long long)((uint32_t)(v >> 32) * mul) << 32);
+            const unsigned long long v = (unsigned long long)X[ch][u][q][e];
+            y[e] = (unsigned long long)(uint32_t)v * mul + off4 + ((unsigned long long)((uint32_t)(v >> 32) * mul) << 32);
           }
           digits(y[0], y[1], [&](int d, uint32_t w) { cd[d][q] = w; });
         }
@@ -370,18 +377,25 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
                 mma(acc[d + j], av[0], av[1], av[2], av[3], cd[j][2 * kt], cd[j][2 * kt + 1]);
             }
           long long *wp = Wp + ((size_t)warp * kCols + 8 * u + 2 * t) * kLdWp + 16 * mt + g;
-          wp[0] = recon<47>(acc, 0, big);
-          wp[kLdWp] = recon<47>(acc, 1, big);
-          wp[8] = recon<47>(acc, 2, big);
-          wp[kLdWp + 8] = recon<47>(acc, 3, big);
+          const long long z0 = recon<47>(acc, 0, big), z1 = recon<47>(acc, 1, big);
+          const long long z2 = recon<47>(acc, 2, big), z3 = recon<47>(acc, 3, big);
+          if (J == 1 || !any) {
+            wp[0] = z0; wp[kLdWp] = z1; wp[8] = z2; wp[kLdWp + 8] = z3;
+          } else {
+            // two shares below 1.25 * 2^62 each: the sum's range is checked on the halves
+            bad |= (int)(((uint64_t)((wp[0] >> 1) + (z0 >> 1) + (1ll << 62)) | (uint64_t)((wp[kLdWp] >> 1) + (z1 >> 1) + (1ll << 62)) |
+                          (uint64_t)((wp[8] >> 1) + (z2 >> 1) + (1ll << 62)) | (uint64_t)((wp[kLdWp + 8] >> 1) + (z3 >> 1) + (1ll << 62))) >> 63);
+            wp[0] += z0; wp[kLdWp] += z1; wp[8] += z2; wp[kLdWp + 8] += z3;
+          }
         }
       }
+      any = true;
     }
     __syncthreads();
     // ---- W1 = A1 rows + the warps' shares ----
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const int q = gtid & 31, c = (gtid >> 5) + 8 * u;
+      const int q = tid & 31, c = (tid >> 5) + 8 * u;
       long long w = 0;
       if (q < kb) {
         int top = 0;
@@ -389,7 +403,9 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
           w = A1s[c * kKMax + i + q];
           top = (int)(w >> 36);
         }
+        const int wlo = J == 1 ? r0 >> 5 : 0, whi = J == 1 ? (Lr + 31) >> 5 : 8;
         for (int ww = wlo; ww < whi; ++ww) {
+          if (J > 1 && !active(0, ww) && !active(1, ww)) continue;
           const uint32_t sh = shw[ww];
           const long long v = (Wp[((size_t)ww * kCols + c) * kLdWp + q] + (long long)sh) >> sh;   // rounded
           w += v;
@@ -436,8 +452,12 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
       }
     }
     __syncthreads();
-    // ---- C -= V W2 on this warp's rows, 8 rows at a time ----
-    if (act) {
+    // ---- C -= V W2 on this warp's rows, 8 rows at a time; the last chunk's digits of V are in place ----
+#pragma unroll
+    for (int cj = 0; cj < J; ++cj) {
+      const int ch = J - 1 - cj;
+      if (!active(ch, warp)) continue;
+      if (J > 1 && cj > 0 && active(J - 1, warp)) v_chunk(ch);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float acc[kD][4];
@@ -459,36 +479,45 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         for (int u = 0; u < 2; ++u)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            X[u][q][e] -= recon<47>(acc, 2 * u + e, big);
-            bad |= (int)((uint32_t)(X[u][q][e] >> 32) >> 31);   // left the biased range
+            const long long dx = recon<47>(acc, 2 * u + e, big);
+            if (J == 1 && dx != 0) changed |= 1u << (8 * u + 2 * q + e);
+            X[ch][u][q][e] -= dx;
+            bad |= (int)((uint32_t)(X[ch][u][q][e] >> 32) >> 31);   // left the biased range
           }
       }
-      if (G == 1) __syncwarp();
+      __syncwarp();
     }
   }
   if (__syncthreads_or(bad | (int)((big & kBig) != 0) | (vmax >= 0x3fff0000u) | (tmax >= 0x400f0000u))) return false;
 
   // ---- back to FP64: the elements whose value changed ----
-  load_c(x);
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
+  for (int ch = 0; ch < J; ++ch) {
+    if (J > 1) load_c(ch, x[ch]);
+    const int rw = 256 * ch + 32 * warp;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = g + 8 * u, r = 32 * warp + 8 * q + 2 * t, s = u ? s1 : s0;
-      double *p = Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs;
-      double y[2];
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const long long v = X[u][q][e] - (long long)kBias;
-        y[e] = v != to_fixed<true>(x[u][q][e], s) ? from_fixed(v, s) : x[u][q][e];
+      for (int q = 0; q < 4; ++q) {
+        const int c = g + 8 * u, r = rw + 8 * q + 2 * t, s = u ? s1 : s0;
+        double *p = Cg + (size_t)r * a.c_rs + (size_t)c * a.c_cs;
+        double y[2];
+        bool moved[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const long long v = X[ch][u][q][e] - (long long)kBias;
+          moved[e] = c < nwl && r + e < Lt &&
+                     (J == 1 ? ((changed >> (8 * u + 2 * q + e)) & 1u) != 0 : v != to_fixed<true>(x[ch][u][q][e], s));
+          y[e] = from_fixed(v, s);
+        }
+        if (vec && moved[0] && moved[1]) {
+          *reinterpret_cast<double2 *>(p) = make_double2(y[0], y[1]);
+        } else {
+          if (moved[0]) p[0] = y[0];
+          if (moved[1]) p[a.c_rs] = y[1];
+        }
       }
-      if (whole) {
-        *reinterpret_cast<double2 *>(p) = make_double2(y[0], y[1]);
-      } else if (c < nwl) {
-        if (r < Lt) p[0] = y[0];
-        if (r + 1 < Lt) p[a.c_rs] = y[1];
-      }
-    }
+  }
 #pragma unroll 4
   for (int r = la; r < ka; r += 16) {
     double *pe = A1g + (size_t)r * a.a_rs;

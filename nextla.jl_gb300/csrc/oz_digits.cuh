@@ -55,9 +55,18 @@ __device__ __forceinline__ long long to_fixed_max(double x, int s, uint32_t &hma
   return to_fixed<false>(x, s);
 }
 
+// v 2^-s rounded to nearest even, |v| < 2^63, the result normal.  On the bits:
+// a conversion instruction would take its warp 64 clocks.
 __device__ __forceinline__ double from_fixed(long long v, int s) {
-  const double d = __ll2double_rn(v);
-  return v == 0 ? 0.0 : __hiloint2double(__double2hiint(d) - (s << 20), __double2loint(d));
+  const unsigned long long sg = (unsigned long long)(v >> 63), a = ((unsigned long long)v ^ sg) - sg;
+  const int lz = __clzll((long long)a);
+  const unsigned long long m = a << lz;                  // leading bit at 63
+  const uint32_t rem = (uint32_t)m & 0x7ffu;
+  unsigned long long q = m >> 11;
+  q += rem + ((uint32_t)q & 1u) > 0x400u ? 1u : 0u;
+  q += (unsigned long long)(unsigned int)(1023 + 62 - lz - s) << 52;   // q's bit 52 adds one to the exponent
+  const uint32_t hi = (uint32_t)(q >> 32) | ((uint32_t)sg & 0x80000000u);
+  return a == 0 ? 0.0 : __hiloint2double((int)hi, (int)(uint32_t)q);
 }
 
 // Digit J (0 = lowest) of two biased fixed-point values as an f16 pair.

@@ -164,6 +164,13 @@ static int cluster_size_for(int mrow, int nc) {
   return mrow >= 192 ? 8 : (mrow >= 96 ? 4 : (mrow >= 64 ? 2 : 0));
 }
 
+// FP64 panels one CTA factors faster with the blocked column loop
+// (panel_blk.cuh) than a cluster does.
+template <typename R>
+static bool blk_panel(int m, int nc) {
+  return std::is_same<R, double>::value && blk::covers(m, nc);
+}
+
 // Launches the cluster panel; *used = false (and nothing launched) when the
 // shape is better left to one CTA or its rows do not fit a cluster of 8.
 template <typename E>
@@ -195,7 +202,7 @@ static cudaError_t launch_cluster(const ClusterPanelArgs<E> &a, int mrow, cudaSt
 
 template <typename R>
 cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt, cudaStream_t st, bool cluster) {
-  if (cluster) {
+  if (cluster && !blk_panel<R>(m, nc)) {
     ClusterPanelArgs<R> a{0, m, nc, A, lda, nullptr, 1, T, ldt, tau, -1};
     bool used = false;
     cudaError_t e = launch_cluster<R>(a, m, st, &used);
@@ -223,7 +230,7 @@ template <typename R>
 cudaError_t launch_tsqrt_block(int m, int sb, R *A1, int lda1, R *A2, int lda2, R *T, int ldt,
                                R *tau, cudaStream_t st, int tt, bool cluster) {
   const int mrow = tt >= 0 ? (m < tt + sb ? m : tt + sb) : m;
-  if (cluster) {
+  if (cluster && !blk_panel<R>(mrow, sb)) {
     ClusterPanelArgs<R> a{1, m, sb, A2, lda2, A1, lda1, T, ldt, tau, tt};
     bool used = false;
     cudaError_t e = launch_cluster<R>(a, mrow, st, &used);

@@ -67,7 +67,8 @@ def worst(x, y, norms):
 
 @pytest.mark.parametrize("m,k,ib,w", [(64, 33, 32, 1), (128, 32, 32, 16), (129, 64, 16, 17), (100, 70, 24, 5),
                                       (255, 256, 32, 31), (256, 256, 32, 48), (121, 35, 17, 16),
-                                      (256, 16, 16, 40), (127, 32, 32, 3)])
+                                      (256, 16, 16, 40), (127, 32, 32, 3), (257, 64, 32, 17),
+                                      (300, 40, 16, 16), (512, 256, 32, 33)])
 def test_tsmqr_every_edge(tq, oracle, m, k, ib, w):
     rng = np.random.default_rng(m + k)
     V, T = reflectors_ts(oracle, m, k, ib, rng)
@@ -88,7 +89,7 @@ def test_tsmqr_every_edge(tq, oracle, m, k, ib, w):
 
 
 @pytest.mark.parametrize("m,k,ib,w", [(128, 32, 32, 3), (130, 40, 16, 16), (256, 200, 32, 33), (200, 199, 31, 16),
-                                      (256, 256, 8, 16)])
+                                      (256, 256, 8, 16), (290, 280, 32, 20), (512, 512, 32, 16), (511, 31, 31, 33)])
 def test_unmqr_every_edge(tq, oracle, m, k, ib, w):
     rng = np.random.default_rng(3 * m + k)
     V, T = reflectors_ge(oracle, m, k, ib, rng)
