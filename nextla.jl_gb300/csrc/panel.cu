@@ -165,7 +165,7 @@ static int cluster_size_for(int mrow, int nc) {
 }
 
 // FP64 panels one CTA factors faster with the blocked column loop
-// (panel_blk.cuh) than a cluster does.
+// (panel_blk.cuh) than a cluster does (256 x 32: 123 against 194 us).
 template <typename R>
 static bool blk_panel(int m, int nc) {
   return std::is_same<R, double>::value && blk::covers(m, nc);

@@ -34,6 +34,7 @@
 #pragma once
 #include "common.cuh"
 #include "panel_blk.cuh"
+#include "panel_reg.cuh"
 
 namespace tqr {
 
@@ -427,6 +428,9 @@ static_assert(8 * ((size_t)(blk::kMaxRows + 1) * 32 + 2 * 33 * 32 + TQR_THREADS 
 
 template <typename R>
 __host__ __device__ inline size_t panel_smem(int m, int nc, bool staged, bool stage_t) {
+  if (std::is_same<R, float>::value && reg::covers(m, nc))
+    return rnd16(sizeof(R) * TQR_THREADS) + rnd16(sizeof(R) * nc) + rnd16(sizeof(R) * 4) +
+           (stage_t ? rnd16(sizeof(R) * (size_t)odd_ld(nc) * nc) : 0) + rnd16(reg::kScratch);
   size_t s = rnd16(sizeof(R) * TQR_THREADS) + rnd16(sizeof(R) * nc) + rnd16(sizeof(R) * 4);
   if (stage_t) s += rnd16(sizeof(R) * (size_t)odd_ld(nc) * nc);
   if (staged) s += rnd16(sizeof(R) * (size_t)odd_ld(m) * nc);
@@ -436,6 +440,9 @@ __host__ __device__ inline size_t panel_smem(int m, int nc, bool staged, bool st
 // (for the ttqrt form pass m = min(m, ii + sb), the rows the block touches)
 template <typename R>
 __host__ __device__ inline size_t tsqrt_smem(int m, int sb, bool staged) {
+  if (std::is_same<R, float>::value && reg::covers(m, sb))
+    return rnd16(sizeof(R) * TQR_THREADS) + rnd16(sizeof(R) * sb) + rnd16(sizeof(R) * 4) +
+           2 * rnd16(sizeof(R) * (size_t)odd_ld(sb) * sb) + rnd16(reg::kScratch);
   size_t s = rnd16(sizeof(R) * TQR_THREADS) + rnd16(sizeof(R) * sb) + rnd16(sizeof(R) * 4) +
              2 * rnd16(sizeof(R) * (size_t)odd_ld(sb) * sb);
   if (staged) s += rnd16(sizeof(R) * (size_t)odd_ld(m) * sb);
@@ -463,6 +470,27 @@ __device__ void panel_qr_cta(int m, int nc, R *A, int lda, R *tau, R *T, int ldt
   } else {
     c.Ts = T;
     c.ldts = ldt;
+  }
+  if constexpr (std::is_same<R, float>::value) {
+    // rows in registers (panel_reg.cuh), scratch where the staged panel would be;
+    // the tensor-core kernels' panels are 32 columns of at most 256 rows
+    if (reg::covers(m, nc) && (!T || stage_t)) {
+      float *scr = carve<float>(sp, reg::kScratch / sizeof(float));
+      if constexpr (VEC) {
+        columns_reg_nc<0, 4, 8>(A, lda, nullptr, 1, c.Ts, c.ldts, m, min(m, nc), nc, -1, true, tau, scr);
+      } else {
+        columns_reg_f32<0>(A, lda, nullptr, 1, c.Ts, c.ldts, m, min(m, nc), nc, -1, true, tau, scr);
+      }
+      if (T) {
+        const int kk = min(m, nc);
+        for (int idx = tid; idx < kk * kk; idx += TQR_THREADS) {
+          const int p = idx % kk, q = idx / kk;
+          if (p <= q) T[ix(p, q, ldt)] = c.Ts[p + (size_t)q * c.ldts];
+        }
+      }
+      __syncthreads();
+      return;
+    }
   }
   if (staged) {
     c.ldp = odd_ld(m);
@@ -560,6 +588,28 @@ __device__ void tsqrt_block_cta(int m, int sb, R *A1, int lda1, R *A2, int lda2,
     if (r <= cc) {
       B[ix(r, cc, ldb)] = ldg_cg(A1 + ix(r, cc, lda1));
       c.Ts[r + (size_t)cc * c.ldts] = ldg_cg(T + ix(r, cc, ldt));   // skipped columns keep T
+    }
+  }
+  if constexpr (std::is_same<R, float>::value) {
+    if (reg::covers(mrow, sb)) {
+      float *scr = carve<float>(sp, reg::kScratch / sizeof(float));
+      __syncthreads();
+      if constexpr (VEC) {
+        if (tt >= 0) columns_reg_nc<2, 4, 8>(A2, lda2, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, false, tau, scr);
+        else columns_reg_nc<1, 4, 8>(A2, lda2, B, ldb, c.Ts, c.ldts, mrow, sb, sb, -1, false, tau, scr);
+      } else {
+        if (tt >= 0) columns_reg_f32<2>(A2, lda2, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, false, tau, scr);
+        else columns_reg_f32<1>(A2, lda2, B, ldb, c.Ts, c.ldts, mrow, sb, sb, -1, false, tau, scr);
+      }
+      for (int idx = tid; idx < sb * sb; idx += TQR_THREADS) {
+        const int r = idx % sb, cc = idx / sb;
+        if (r <= cc) {
+          A1[ix(r, cc, lda1)] = B[ix(r, cc, ldb)];
+          T[ix(r, cc, ldt)] = c.Ts[r + (size_t)cc * c.ldts];
+        }
+      }
+      __syncthreads();
+      return;
     }
   }
   if (staged) {
