@@ -17,6 +17,9 @@
 // the next task index from a global counter, waits until the task's inputs
 // are written, runs it, and publishes its writes by bumping counters:
 //   ver(i,j,s)   number of completed tasks that wrote strip s of tile (i,j)
+//                (the diagonal tile: geqrt's own)
+//   lead(k,b,s)  those that wrote row block b of strip s of the diagonal tile,
+//                the part of it that block b of geqrt and of every tsqrt touches
 //   done_g(k)    completed GB/GA tasks of diagonal tile k
 //   done_t(k,i)  completed TB/TA tasks of tsqrt(k,i)
 // Every writer of a strip is known in advance, so a task's wait targets are
@@ -82,7 +85,11 @@ struct DagGeom {
   __host__ __device__ int ver(int i, int j, int s) const { return (i * NT + j) * NS + s; }
   __host__ __device__ int done_g(int k) const { return MT * NT * NS + k; }
   __host__ __device__ int done_t(int k, int i) const { return MT * NT * NS + KT + k * MT + i; }
-  __host__ __device__ int ncounters() const { return MT * NT * NS + KT + KT * MT; }
+  // row block b of strip s of the diagonal tile (k, k), which the tsqrts of
+  // panel k update one after another: a counter of its own, so that tile i + 1
+  // follows tile i block by block and does not wait for i's later blocks
+  __host__ __device__ int lead(int k, int b, int s) const { return MT * NT * NS + KT + KT * MT + (k * NBK + b) * NS + s; }
+  __host__ __device__ int ncounters() const { return MT * NT * NS + KT + KT * MT + KT * NBK * NS; }
   // tasks of one geqrt (GB + GA) or one tsqrt (TB + TA)
   __host__ __device__ int panel_tasks() const { return NBK + NBK * NS - SPB * NBK * (NBK + 1) / 2; }
 };
@@ -106,19 +113,15 @@ __host__ __device__ inline int item_deps(const DagGeom &g, const DagItem &it, in
       c[n] = g.ver(k, j, s); t[n++] = k;
       break;
     case IT_TB:
-      // (k,k): geqrt and each earlier tsqrt wrote b+1 times, this tsqrt b times
-      for (int q = b * g.SPB; q < (b + 1) * g.SPB; ++q) {
-        c[n] = g.ver(k, k, q); t[n++] = k + (i - k) * (b + 1) + b;
-        c[n] = g.ver(i, k, q); t[n++] = k + b;
-      }
+      // the diagonal block: geqrt's block and each earlier tsqrt's wrote it once
+      c[n] = g.lead(k, b, b * g.SPB); t[n++] = i - k;
+      for (int q = b * g.SPB; q < (b + 1) * g.SPB; ++q) { c[n] = g.ver(i, k, q); t[n++] = k + b; }
       break;
-    case IT_TA: {
-      const int bs = s / g.SPB;
-      c[n] = g.ver(k, k, s); t[n++] = k + (i - k) * (bs + 1) + b;
+    case IT_TA:
+      c[n] = g.lead(k, b, s); t[n++] = i - k;
       c[n] = g.ver(i, k, s); t[n++] = k + b;
       c[n] = g.ver(i, k, b * g.SPB); t[n++] = k + b + 1;
       break;
-    }
     case IT_TM:
       c[n] = g.done_t(k, i); t[n++] = g.panel_tasks();
       c[n] = g.ver(k, j, s); t[n++] = i;
@@ -141,11 +144,15 @@ __host__ __device__ inline int item_updates(const DagGeom &g, const DagItem &it,
   const int k = it.k, i = it.i, j = it.j, b = it.b, s = it.s;
   switch (it.type) {
     case IT_GB:
-      for (int q = b * g.SPB; q < (b + 1) * g.SPB; ++q) c[n++] = g.ver(k, k, q);
+      for (int q = b * g.SPB; q < (b + 1) * g.SPB; ++q) {
+        c[n++] = g.ver(k, k, q);
+        c[n++] = g.lead(k, b, q);
+      }
       c[n++] = g.done_g(k);
       break;
     case IT_GA:
       c[n++] = g.ver(k, k, s);
+      c[n++] = g.lead(k, b, s);
       c[n++] = g.done_g(k);
       break;
     case IT_UN:
@@ -153,13 +160,13 @@ __host__ __device__ inline int item_updates(const DagGeom &g, const DagItem &it,
       break;
     case IT_TB:
       for (int q = b * g.SPB; q < (b + 1) * g.SPB; ++q) {
-        c[n++] = g.ver(k, k, q);
+        c[n++] = g.lead(k, b, q);
         c[n++] = g.ver(i, k, q);
       }
       c[n++] = g.done_t(k, i);
       break;
     case IT_TA:
-      c[n++] = g.ver(k, k, s);
+      c[n++] = g.lead(k, b, s);
       c[n++] = g.ver(i, k, s);
       c[n++] = g.done_t(k, i);
       break;
@@ -900,7 +907,8 @@ static int tile_geqrf_dag(int m, int n, int nb, int ib, R *A, int lda, R *T, int
 // neither the host nor the device allocates anything per call.
 // ---------------------------------------------------------------------------
 constexpr size_t kStaticScratchBytes = size_t(4) << 20;   // 4 MiB (see tileqr.h)
-static __device__ __align__(256) unsigned char g_tile_scratch[kStaticScratchBytes];
+// plus the lead counters: at most one per two panel tasks (12 bytes each)
+static __device__ __align__(256) unsigned char g_tile_scratch[kStaticScratchBytes + (size_t(3) << 20)];
 
 static std::mutex g_static_mu;
 static void *g_static_ptr[64];
@@ -969,7 +977,9 @@ static int tile_geqrf_noalloc(int m, int n, int nb, int ib, double *A, int lda, 
   for (int k = 0; k < g.KT; ++k) nitems += step_tasks(g, k);
   const size_t bytes_counters = align256(sizeof(int) * (size_t)g.ncounters());
   const size_t need = 256 + bytes_counters + sizeof(DagItem) * (size_t)nitems;
-  if (need > kStaticScratchBytes || nitems > 0x7fffffff) return TQR_ERR_SCRATCH_TOO_SMALL;
+  const size_t lead_bytes = sizeof(int) * (size_t)g.KT * g.NBK * g.NS;
+  if (need - lead_bytes > kStaticScratchBytes || need > sizeof(g_tile_scratch) || nitems > 0x7fffffff)
+    return TQR_ERR_SCRATCH_TOO_SMALL;
   void *wv = nullptr;
   cudaError_t e = static_scratch(&wv);
   if (e != cudaSuccess) return (int)e;

@@ -799,7 +799,13 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
   // compact-WY slots (wy_slot), after the T blocks
   const size_t nslot_reg = nstrip + (size_t)sh.MT * sh.KT * nblk * 2;
   auto rs = [&](int merge, int row, int k) { return nslot_reg + (size_t)wy_slot(sh.MT, merge, row, k); };
-  const size_t nreg = nslot_reg + (size_t)4 * sh.MT;
+  // row block b of strip q of tile (i, k) as the leader of panel k's merges:
+  // block b of geqrt finishes it, block b of every merge into the tile updates
+  // it, so the merges follow one another block by block; a partner of a ttqrt
+  // merge gives its row blocks 0 .. b to block b
+  const size_t nlead_reg = nslot_reg + (size_t)4 * sh.MT;
+  auto rl = [&](int i, int k, int b, int q) { return nlead_reg + (((size_t)i * sh.KT + k) * nblk + b) * NS + q; };
+  const size_t nreg = nlead_reg + (size_t)sh.MT * sh.KT * nblk * NS;
   std::vector<int> last(nreg, -1);
   std::vector<std::vector<int>> readers(nreg);
   std::vector<TItem> items;
@@ -851,7 +857,7 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
       for (int b = 0, c = 0; c < kk; ++b, c += sh.ib) {
         const int sb = std::min(sh.ib, kk - c);
         const int q0 = c / sh.nw, q1 = (c + sb + sh.nw - 1) / sh.nw;
-        for (int q = q0; q < q1; ++q) { wr(rg(i, k, q, 0)); wr(rg(i, k, q, 1)); }
+        for (int q = q0; q < q1; ++q) { wr(rg(i, k, q, 0)); wr(rg(i, k, q, 1)); wr(rl(i, k, b, q)); }
         wr(rt(i, k, b, 0));
         emit(OP_GE_PANEL, k, b, i, i, 0);
         // strip y covers columns [c + sb + 16 y, +16) clipped to nk (as in tree_task)
@@ -859,7 +865,9 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
           const int c0 = c + sb + y * sh.nw, c1 = std::min(nk, c0 + sh.nw);
           for (int v = q0; v < q1; ++v) rd(rg(i, k, v, 1));
           rd(rt(i, k, b, 0));
-          for (int q = c0 / sh.nw; q <= (c1 - 1) / sh.nw; ++q) { wr(rg(i, k, q, 0)); wr(rg(i, k, q, 1)); }
+          for (int q = c0 / sh.nw; q <= (c1 - 1) / sh.nw; ++q) {
+            wr(rg(i, k, q, 0)); wr(rg(i, k, q, 1)); wr(rl(i, k, b, q));
+          }
           emit(OP_GE_APPLY, k, b, i, i, y);
         }
       }
@@ -901,27 +909,36 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
     auto merge = [&](int i, int p, int ts) {
       const int kt = ts ? nk : std::min(sh.rows(p), nk);
       const int flag = ts ? 0x80 : 0;
+      // strip q of the partner as block b touches it: the whole strip of a
+      // tsqrt partner (no leader), row blocks 0 .. b of a ttqrt partner (a leader)
+      auto wr_partner = [&](int b, int q) {
+        if (ts) { wr(rg(p, k, q, 0)); wr(rg(p, k, q, 1)); return; }
+        for (int b2 = 0; b2 <= b; ++b2) wr(rl(p, k, b2, q));
+      };
+      auto rd_partner = [&](int b, int q) {
+        if (ts) { rd(rg(p, k, q, 0)); rd(rg(p, k, q, 1)); return; }
+        for (int b2 = 0; b2 <= b; ++b2) rd(rl(p, k, b2, q));
+      };
+      // all of the partner's reflectors
+      auto rd_reflectors = [&]() {
+        for (int q = 0; q < NSk; ++q) rd_partner(std::min(nblk - 1, q * sh.nw / sh.ib), q);
+      };
       for (int b = 0, c = 0; c < kt; ++b, c += sh.ib) {
         const int sb = std::min(sh.ib, kt - c);
         const int q0 = c / sh.nw, q1 = (c + sb + sh.nw - 1) / sh.nw;
         for (int q = q0; q < q1; ++q) {
-          wr(rg(i, k, q, 0));
-          wr(rg(p, k, q, 0));
-          if (ts) wr(rg(p, k, q, 1));
+          wr(rl(i, k, b, q));
+          wr_partner(b, q);
         }
         wr(rt(p, k, b, 1));
         emit(OP_PR_PANEL | flag, k, b, i, p, 0);
         for (int y = 0; c + sb + y * sh.nw < nk; ++y) {
           const int c0 = c + sb + y * sh.nw, c1 = std::min(nk, c0 + sh.nw);
-          for (int v = q0; v < q1; ++v) {
-            rd(rg(p, k, v, 0));
-            if (ts) rd(rg(p, k, v, 1));
-          }
+          for (int v = q0; v < q1; ++v) rd_partner(b, v);
           rd(rt(p, k, b, 1));
           for (int q = c0 / sh.nw; q <= (c1 - 1) / sh.nw; ++q) {
-            wr(rg(i, k, q, 0));
-            wr(rg(p, k, q, 0));
-            if (ts) wr(rg(p, k, q, 1));
+            wr(rl(i, k, b, q));
+            wr_partner(b, q);
           }
           emit(OP_PR_APPLY | flag, k, b, i, p, y);
         }
@@ -934,10 +951,7 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
       if (sh.tc && sh.rows(p) == sh.nb && sh.rows(i) == sh.nb && kt == sh.nb && ca % tc::kChunk == 0) {
         if (sh.wy && ca > 0) {
           // the slot of the merge's V and T for the chunks below
-          for (int q = 0; q < NSk; ++q) {
-            rd(rg(p, k, q, 0));
-            if (ts) rd(rg(p, k, q, 1));
-          }
+          rd_reflectors();
           for (int b = 0; b < nbk; ++b) rd(rt(p, k, b, 1));
           wr(rs(1, p, k));
           emit(OP_WY_BUILD | flag, k, 1, i, p, 0);
@@ -946,10 +960,7 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
           if (sh.wy) {
             rd(rs(1, p, k));
           } else {
-            for (int q = 0; q < NSk; ++q) {
-              rd(rg(p, k, q, 0));
-              if (ts) rd(rg(p, k, q, 1));
-            }
+            rd_reflectors();
             for (int b = 0; b < nbk; ++b) rd(rt(p, k, b, 1));
           }
           const int c0 = ch * tc::kChunk, j = k + 1 + c0 / sh.nb, s0 = (c0 % sh.nb) / sh.nw;
@@ -964,10 +975,7 @@ static void tree_build(const TreeShape &sh, std::vector<TItem> &out_items, std::
       for (int y = y0; y < ntrail(k); ++y) {
         int j, s;
         trail_js(k, y, j, s);
-        for (int q = 0; q < NSk; ++q) {
-          rd(rg(p, k, q, 0));
-          if (ts) rd(rg(p, k, q, 1));
-        }
+        rd_reflectors();
         for (int b = 0; b < nbk; ++b) rd(rt(p, k, b, 1));
         wr(rg(i, j, s, 0)); wr(rg(i, j, s, 1));
         wr(rg(p, j, s, 0)); wr(rg(p, j, s, 1));
