@@ -57,7 +57,8 @@ struct BatchHeader {           // first 256 bytes of the workspace
   int next;                    // problem counter (cleared before every launch)
   int bad;                     // descriptors rejected by the kernel
   int first_bad;               // smallest rejected problem index (INT_MAX if none)
-  int pad[61];
+  int next_oz;                 // problem counter of the tensor-core pass (double precision)
+  int pad[60];
 };
 static_assert(sizeof(BatchHeader) == 256, "BatchHeader layout");
 
@@ -99,7 +100,7 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
     a.V = A + ix(i, i, lda); a.ldv = lda;
     a.T = Tscr; a.ldt = ib;
     a.stage_t = 1;
-    const int nw = p.nw;
+    const int nw = OZ ? 16 : p.nw;     // the tensor-core strips are 16 columns, whatever the loops prefer
     constexpr size_t cap = OZ ? oz::kSmem : kBatchSmem;
     const bool full = apply_smem_elems(L, sb, nw, true, true, true) * sizeof(R) <= cap;
     a.stage_v = full;
@@ -140,43 +141,65 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
   __syncthreads();
 }
 
-template <typename R> constexpr bool kBatchOz = std::is_same<R, double>::value;
-template <typename R> constexpr size_t kBatchDynSmem = kBatchOz<R> ? oz::kSmem : kBatchSmem;
+// FP64 problems that a CTA with the SM to itself solves faster, on the
+// tensor-core paths, than two CTAs per SM do on the FP64 loops (2000 equal
+// problems, ms: 256 x 64 5.5 against 7.7, 192 x 150 16.5 against 23.5; 128 x 64
+// 5.05 against 5.01, 128 x 120 13.8 against 12.6, 192 x 32 2.9 against 2.8,
+// 64 x 32 2.8 against 1.7).
+__host__ __device__ inline bool batch_oz(int m, int n) { return m > 128 && n > 32; }
+
+template <bool OZ> constexpr size_t kBatchDynSmem = OZ ? oz::kSmem : kBatchSmem;
 static_assert(sizeof(double) * ((size_t)513 * 32 + 33 * 32 + TQR_THREADS + 64) + blk::kScratch <= oz::kSmem,
               "a staged 512-row panel with the blocked loop's scratch");
 
-template <typename R>
-__global__ void __launch_bounds__(TQR_THREADS, kBatchOz<R> ? 1 : 2)
+// One pass over the batch.  Double precision takes two: OZ, the problems of
+// batch_oz; not OZ, the others (every other element type: all of them).  A CTA
+// takes one problem at a time; after one that is not its own it looks at up
+// to 32 at once.
+template <typename R, bool OZ>
+__global__ void __launch_bounds__(TQR_THREADS, OZ ? 1 : 2)
 k_batched_gels(int nprob, const BatchProblem *__restrict__ probs, const int *__restrict__ order, R *A, R *B,
                BatchHeader *hdr, R *scratch)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_q;
+  __shared__ unsigned s_mine;
   R *Tscr = scratch + (size_t)blockIdx.x * kScrElems;
   R *tauscr = Tscr + kBatchMaxIb * kBatchMaxIb;
+  constexpr bool kSplit = std::is_same<R, double>::value;
+  int *const next = OZ ? &hdr->next_oz : &hdr->next;
+  int take = 1;
   for (;;) {
-    if (threadIdx.x == 0) s_q = atomicAdd(&hdr->next, 1);
-    __syncthreads();
-    const int q = s_q;
-    __syncthreads();
-    if (q >= nprob) break;
-    const int id = order[q];
-    if (id < 0 || id >= nprob) {
-      if (threadIdx.x == 0) { atomicAdd(&hdr->bad, 1); atomicMin(&hdr->first_bad, q); }
-      continue;
+    if (threadIdx.x < 32) {
+      int q0 = 0;
+      if (threadIdx.x == 0) q0 = atomicAdd(next, take);
+      q0 = __shfl_sync(0xffffffffu, q0, 0);
+      const int q = q0 + (int)threadIdx.x;
+      bool mine = false;
+      if ((int)threadIdx.x < take && q < nprob) {
+        const int id = order[q];
+        const bool known = id >= 0 && id < nprob;
+        const bool ok = known && problem_ok(probs[id]);
+        mine = ok && (!kSplit || batch_oz(probs[id].m, probs[id].n) == OZ);
+        if (!ok && !OZ) { atomicAdd(&hdr->bad, 1); atomicMin(&hdr->first_bad, known ? id : q); }
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, mine);
+      if (threadIdx.x == 0) { s_q = q0; s_mine = mask; }
     }
-    const BatchProblem p = probs[id];
-    if (!problem_ok(p)) {
-      if (threadIdx.x == 0) { atomicAdd(&hdr->bad, 1); atomicMin(&hdr->first_bad, id); }
-      continue;
-    }
-    solve_one<R, kBatchOz<R>>(p, A, B, Tscr, tauscr, smem_raw);
+    __syncthreads();
+    const int q0 = s_q;
+    unsigned mine = s_mine;
+    __syncthreads();
+    if (q0 >= nprob) break;
+    take = kSplit && mine == 0 ? min(32, 2 * take) : 1;
+    for (; mine; mine &= mine - 1) solve_one<R, OZ>(probs[order[q0 + __ffs(mine) - 1]], A, B, Tscr, tauscr, smem_raw);
   }
 }
 
 __global__ void k_batch_reset(BatchHeader *hdr) {
   if (threadIdx.x == 0) {
     hdr->next = 0;
+    hdr->next_oz = 0;
     hdr->bad = 0;
     hdr->first_bad = 0x7fffffff;
   }
@@ -185,7 +208,8 @@ __global__ void k_batch_reset(BatchHeader *hdr) {
 // Launch shape per device and precision, fixed on first use (before any
 // capture): grid = resident CTAs per SM x SMs.
 struct LaunchCfg {
-  int grid = 0;
+  int grid = 0;                // of the pass every element type has
+  int grid_oz = 0;             // of the tensor-core pass
   cudaError_t err = cudaSuccess;
 };
 static std::mutex g_cfg_mu;
@@ -194,6 +218,17 @@ static LaunchCfg g_cfg[4][64];
 // Launch-shape slot of an element type: double, float, ComplexF64, ComplexF32.
 template <typename R> constexpr int cfg_slot() {
   return std::is_same<R, double>::value ? 0 : std::is_same<R, float>::value ? 1 : std::is_same<R, cx<double>>::value ? 2 : 3;
+}
+
+template <typename R, bool OZ>
+static cudaError_t pass_grid(int sms, int *grid) {
+  int per_sm = 0;
+  cudaError_t e = cudaFuncSetAttribute(k_batched_gels<R, OZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kBatchDynSmem<OZ>);
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_gels<R, OZ>, TQR_THREADS, kBatchDynSmem<OZ>);
+  if (e == cudaSuccess) *grid = sms * std::max(per_sm, 1);
+  return e;
 }
 
 template <typename R>
@@ -205,15 +240,13 @@ static LaunchCfg launch_cfg() {
   std::lock_guard<std::mutex> l(g_cfg_mu);
   LaunchCfg &g = g_cfg[cfg_slot<R>()][dev];
   if (g.grid > 0) return g;
-  int sms = 0, per_sm = 0;
+  int sms = 0;
   if ((c.err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return c;
-  if ((c.err = cudaFuncSetAttribute(k_batched_gels<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)kBatchDynSmem<R>)) != cudaSuccess)
-    return c;
-  if ((c.err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batched_gels<R>, TQR_THREADS,
-                                                             kBatchDynSmem<R>)) != cudaSuccess)
-    return c;
-  g.grid = sms * std::max(per_sm, 1);
+  if ((c.err = pass_grid<R, false>(sms, &c.grid)) != cudaSuccess) return c;
+  if constexpr (std::is_same<R, double>::value) {
+    if ((c.err = pass_grid<R, true>(sms, &c.grid_oz)) != cudaSuccess) return c;
+  }
+  g = c;
   return g;
 }
 
@@ -239,9 +272,13 @@ static int batched_launch(int nprob, const void *probs, const int *order, R *A, 
   k_batch_reset<<<1, 32, 0, st>>>(hdr);
   count_launch();
   if (nprob > 0) {
-    const int grid = std::min(c.grid, nprob);
-    k_batched_gels<R><<<grid, TQR_THREADS, kBatchDynSmem<R>, st>>>(nprob, (const BatchProblem *)probs, order, A, B,
-                                                             hdr, scratch);
+    if constexpr (std::is_same<R, double>::value) {
+      k_batched_gels<R, true><<<std::min(c.grid_oz, nprob), TQR_THREADS, kBatchDynSmem<true>, st>>>(
+          nprob, (const BatchProblem *)probs, order, A, B, hdr, scratch);
+      count_launch();
+    }
+    k_batched_gels<R, false><<<std::min(c.grid, nprob), TQR_THREADS, kBatchDynSmem<false>, st>>>(
+        nprob, (const BatchProblem *)probs, order, A, B, hdr, scratch);
     count_launch();
   }
   cudaError_t e = cudaGetLastError();
@@ -366,7 +403,7 @@ static int autotune(cudaStream_t st, int force) {
   LaunchCfg c = launch_cfg<R>();
   if (c.err != cudaSuccess) return (int)c.err;
   // class representatives (m, n) and candidate (ib, nw)
-  const int shape[kClasses][2] = {{64, 24}, {160, 48}, {256, 96}, {384, 192}, {512, 384}};
+  const int shape[kClasses][2] = {{64, 24}, {112, 48}, {256, 96}, {384, 192}, {512, 384}};
   const Tune cand[6] = {{8, 8}, {16, 8}, {16, 16}, {32, 8}, {32, 16}, {24, 16}};
   const int kr = 4;
   const int np = 2 * c.grid;   // two waves of the persistent grid
