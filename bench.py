@@ -1478,16 +1478,28 @@ def main():
             traffic = json.load(open(tpath)).get("bytes_per_launch")
         except (OSError, ValueError):
             traffic = None
-    roofline = {"bound": "fp64_simt", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": (achieved / peak) if achieved else None, "traffic": traffic,
+    # the trailing updates run as 28 exact FP16 tensor-core products per FP64
+    # product: the ceiling is the half-precision tensor rate over 28
+    half_peak = 1900.0
+    ppath = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    if os.path.exists(ppath):
+        try:
+            half_peak = float(json.load(open(ppath))["bf16_tflops"])
+        except (OSError, ValueError, KeyError, TypeError):
+            pass
+    split_peak = half_peak / 28.0
+    roofline = {"bound": "fp16_tensor_exact_split", "achieved": achieved, "peak": split_peak, "unit": "TFLOP/s",
+                "frac": (achieved / split_peak) if achieved else None, "traffic": traffic,
+                "fp64_simt_tflops": peak, "frac_of_fp64_simt": (achieved / peak) if achieved else None,
                 "fp64_mma_tflops": mma_peak,
                 "frac_of_fp64_mma": (achieved / mma_peak) if (achieved and mma_peak) else None,
                 "cublas_dgemm_tflops": dgemm,
                 "fp64_mma_dfma_mix": mma_mix,
                 "kernel": ("k_tile_dag (one persistent launch per factorisation: panel, unmqr and "
-                           "tsmqr tasks), FP64 SIMT DFMA; algorithmic flops 4/3 n^3 per launch"),
-                "peak_source": ("measured live: DFMA-chain probe (tqr_fp64_peak_probe), the FP64 ceiling "
-                                "on this GPU; the FP64 tensor-core rate (tqr_fp64_mma_probe, "
+                           "tsmqr tasks), updates by exact FP16 digit products; algorithmic flops 4/3 n^3 per launch"),
+                "peak_source": ("half-precision tensor rate (MEASURED_PEAKS.json bf16_tflops, else 1900) over 28 "
+                                "digit products; beside it, measured live: DFMA-chain probe "
+                                "(tqr_fp64_peak_probe), the FP64 tensor-core rate (tqr_fp64_mma_probe, "
                                 "mma.sync.m8n8k4.f64) and cuBLAS DGEMM measured alongside; "
                                 "MEASURED_PEAKS.json has no FP64 figure"),
                 "timed_launches": prof_n, "algorithmic_flops_per_launch": (prof_flops / prof_n) if prof_n else None,

@@ -24,6 +24,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <numeric>
 #include <type_traits>
@@ -465,6 +466,10 @@ static int autotune(cudaStream_t st, int force) {
   return rc;
 }
 
+// kernels of each instantiated graph, for the launch count
+static std::mutex g_graph_mu;
+static std::map<void *, int> g_graph_kernels;
+
 }  // namespace tqr
 
 using namespace tqr;
@@ -616,19 +621,31 @@ int tqr_batched_graph(int dtype_bytes, int nprob, const void *problems, const in
   }
   if (g) cudaGraphDestroy(g);
   cudaStreamDestroy(s);
-  if (rc == 0) *graph_exec = (void *)ex;
+  if (rc == 0) {
+    *graph_exec = (void *)ex;
+    std::lock_guard<std::mutex> l(g_graph_mu);
+    g_graph_kernels[*graph_exec] = dtype_bytes == 8 ? 3 : 2;   // reset and the passes
+  }
   return rc;
 }
 
 int tqr_batched_graph_launch(void *graph_exec, cudaStream_t stream) {
   if (!graph_exec) return -1;
   cudaError_t e = cudaGraphLaunch((cudaGraphExec_t)graph_exec, stream);
-  if (e == cudaSuccess) count_launch(2);
+  if (e == cudaSuccess) {
+    std::lock_guard<std::mutex> l(g_graph_mu);
+    const auto f = g_graph_kernels.find(graph_exec);
+    count_launch(f == g_graph_kernels.end() ? 2 : f->second);
+  }
   return e == cudaSuccess ? 0 : (int)e;
 }
 
 int tqr_batched_graph_destroy(void *graph_exec) {
   if (!graph_exec) return 0;
+  {
+    std::lock_guard<std::mutex> l(g_graph_mu);
+    g_graph_kernels.erase(graph_exec);
+  }
   cudaError_t e = cudaGraphExecDestroy((cudaGraphExec_t)graph_exec);
   return e == cudaSuccess ? 0 : (int)e;
 }

@@ -137,25 +137,32 @@ __device__ __forceinline__ void columns_reg_nc(float *A, int lda, float *B, int 
       }
 #pragma unroll
       for (int u = 0; u < CPW; ++u) a[u] = lanes(a[u], x0);
+      // d of the warp's columns, side by side, then their updates
+      float d[CPW], rv[CPW];
 #pragma unroll
       for (int u = 0; u < CPW; ++u) {
         const int j = 8 * u + warp;
-        if (j == i || j >= nc) continue;
-        float s = a[u];
-        float *const row = B + i + (size_t)j * ldb;
-        const float rv = FORM == 0 ? __shfl_sync(kAll, x[u][0], i) : (j > i ? *row : 0.0f);
-        if (FORM == 0 || j > i) s += rv;
-        const float d = -(tv * s);
-        if (lane == 0) ds[j] = d;
-        if (j > i) {
+        rv[u] = FORM == 0 ? __shfl_sync(kAll, x[u][0], i) : (j > i && j < nc ? B[i + (size_t)j * ldb] : 0.0f);
+      }
 #pragma unroll
-          for (int t = 1; t < RPL; ++t) x[u][t] = fmaf(v[t], d, x[u][t]);
-          if (on0) x[u][0] = fmaf(v[0], d, x[u][0]);
-          if (FORM == 0 && lane == i) x[u][0] += d;
-          if (FORM != 0) {
-            __syncwarp();                                 // every lane has the row's entry
-            if (lane == 0) *row = rv + d;
-          }
+      for (int u = 0; u < CPW; ++u) {
+        const int j = 8 * u + warp;
+        const float s = FORM == 0 || j > i ? a[u] + rv[u] : a[u];
+        d[u] = -(tv * s);
+      }
+      if (FORM != 0) __syncwarp();                        // every lane has the rows' entries
+#pragma unroll
+      for (int u = 0; u < CPW; ++u) {
+        const int j = 8 * u + warp;
+        if (lane == 0 && j != i && j < nc) {
+          ds[j] = d[u];
+          if (FORM != 0 && j > i) B[i + (size_t)j * ldb] = rv[u] + d[u];
+        }
+        if (j > i && j < nc) {
+#pragma unroll
+          for (int t = 1; t < RPL; ++t) x[u][t] = fmaf(v[t], d[u], x[u][t]);
+          if (on0) x[u][0] = fmaf(v[0], d[u], x[u][0]);
+          if (FORM == 0 && lane == i) x[u][0] += d[u];
         }
       }
     }
