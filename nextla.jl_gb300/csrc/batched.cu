@@ -193,7 +193,10 @@ k_batched_gels(int nprob, const BatchProblem *__restrict__ probs, const int *__r
     __syncthreads();
     if (q0 >= nprob) break;
     take = kSplit && mine == 0 ? min(32, 2 * take) : 1;
-    for (; mine; mine &= mine - 1) solve_one<R, OZ>(probs[order[q0 + __ffs(mine) - 1]], A, B, Tscr, tauscr, smem_raw);
+    for (; mine; mine &= mine - 1) {
+      const BatchProblem p = probs[order[q0 + __ffs(mine) - 1]];
+      solve_one<R, OZ>(p, A, B, Tscr, tauscr, smem_raw);
+    }
   }
 }
 
@@ -404,7 +407,7 @@ static int autotune(cudaStream_t st, int force) {
   LaunchCfg c = launch_cfg<R>();
   if (c.err != cudaSuccess) return (int)c.err;
   // class representatives (m, n) and candidate (ib, nw)
-  const int shape[kClasses][2] = {{64, 24}, {112, 48}, {256, 96}, {384, 192}, {512, 384}};
+  const int shape[kClasses][2] = {{64, 24}, {160, 48}, {256, 96}, {384, 192}, {512, 384}};
   const Tune cand[6] = {{8, 8}, {16, 8}, {16, 16}, {32, 8}, {32, 16}, {24, 16}};
   const int kr = 4;
   const int np = 2 * c.grid;   // two waves of the persistent grid

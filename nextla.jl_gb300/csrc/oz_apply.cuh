@@ -15,8 +15,8 @@
 // Number format.  Column c of [A1; C] is held as 64-bit fixed point with its
 // own power-of-two scale 2^s: s is the largest with ||column|| 2^s <= 2^60.9.
 // An orthogonal update keeps that norm, |W| <= 2 ||column||, so nothing leaves
-// the 62-bit range the digits cover; V (|v| < 1.93) is scaled by 2^61 and T
-// (|t| < 3.87) by 2^60.  A strip that is not such an update (an infinity or NaN,
+// the 62-bit range the digits cover; V (|v| < 1.99) is scaled by 2^61 and T
+// (|t| < 3.99) by 2^60.  A strip that is not such an update (an infinity or NaN,
 // exponents near the ends of the range, a V or T beyond those bounds, a sum
 // that overflows) is detected before anything is written and the caller runs
 // the DFMA path on it.  An element whose fixed-point value the update did not
@@ -131,7 +131,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   const bool tt = a.mode == 1 && a.tt >= 0;
   const int Lt = tt ? min(L, a.tt + k) : L;            // rows any reflector touches
   int bad = 0;
-  uint32_t big = 0, vmax = 0, tmax = 0;
+  uint32_t big = 0, vout = 0;                          // vout: top bit set by a V or T out of range
 
   // ---- the strip, and A1's rows, from global memory ----
   double *const Cg = a.C + (size_t)c0 * a.c_cs;
@@ -172,7 +172,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   const int ka = a.mode == 1 && ca < nwl ? k : 0;
   double *const A1c = reinterpret_cast<double *>(A1s) + ca * kKMax;
   uint32_t m0 = 0, m1 = 0, ma = 0;
-#pragma unroll 4
+#pragma unroll 8
   for (int r = la; r < ka; r += 16) {
     const double v = __ldcg(A1g + (size_t)r * a.a_rs);
     A1c[r] = v;
@@ -305,8 +305,8 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         if (p + kStep < np) load_v(a, Vg, wholev, r, p + kStep, kb, i, Lr, tt, n);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          const unsigned long long y0 = (unsigned long long)to_fixed_max(v[u][0], 61, vmax) + kBias;
-          const unsigned long long y1 = (unsigned long long)to_fixed_max(v[u][1], 61, vmax) + kBias;
+          const unsigned long long y0 = to_biased<61>(v[u][0], vout);
+          const unsigned long long y1 = to_biased<61>(v[u][1], vout);
           const uint32_t off = plane_off(p + 2 * u, 2 * (lane & 15));
           digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Vd + d * kPlaneV + off) = w; });
         }
@@ -321,8 +321,8 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
         const int idx = tid + w * TQR_THREADS, p = idx >> 4, q = 2 * (idx & 15);
-        const unsigned long long y0 = (unsigned long long)to_fixed_max(tv[w][0], 60, tmax) + kBias;
-        const unsigned long long y1 = (unsigned long long)to_fixed_max(tv[w][1], 60, tmax) + kBias;
+        const unsigned long long y0 = to_biased<60>(tv[w][0], vout);
+        const unsigned long long y1 = to_biased<60>(tv[w][1], vout);
         const uint32_t off = plane_off(p, q);
         digits(y0, y1, [&](int d, uint32_t z) { *reinterpret_cast<uint32_t *>(Td + d * kPlaneV + off) = z; });
       }
@@ -488,7 +488,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
       __syncwarp();
     }
   }
-  if (__syncthreads_or(bad | (int)((big & kBig) != 0) | (vmax >= 0x3fff0000u) | (tmax >= 0x400f0000u))) return false;
+  if (__syncthreads_or(bad | (int)((big & kBig) != 0) | (int)(vout >> 31))) return false;
 
   // ---- back to FP64: the elements whose value changed ----
 #pragma unroll
@@ -518,7 +518,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         }
       }
   }
-#pragma unroll 4
+#pragma unroll 8
   for (int r = la; r < ka; r += 16) {
     double *pe = A1g + (size_t)r * a.a_rs;
     const double o = __ldcg(pe);

@@ -49,10 +49,18 @@ __device__ __forceinline__ long long to_fixed(double x, int s) {
   const long long sg = (long long)((int)hi >> 31);
   return ((long long)m ^ sg) - sg;
 }
-// the same, with the largest high word of |x| collected for a bound check
-__device__ __forceinline__ long long to_fixed_max(double x, int s, uint32_t &hmax) {
-  hmax = max(hmax, (uint32_t)__double2hiint(x) & 0x7fffffffu);
-  return to_fixed<false>(x, s);
+// x 2^S biased by kBias, towards zero; out's top bit is set if some x was out
+// of the digits' range (0.998 * 2^62 and up, infinities, NaN).
+template <int S>
+__device__ __forceinline__ unsigned long long to_biased(double x, uint32_t &out) {
+  const uint32_t hi = __double2hiint(x), lo = __double2loint(x);
+  const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32 | lo) << 10;
+  const int t = (1085 - S) - (int)((hi & 0x7fffffffu) >> 20);
+  const unsigned long long r = m >> min(max(t, 0), 63);  // 63 leaves nothing
+  const uint32_t sg = (uint32_t)((int)hi >> 31);
+  const unsigned long long y = (r ^ ((unsigned long long)sg << 32 | sg)) + ((kBias & 0xffffffff00000000ull) | ((uint32_t)kBias - sg));
+  out |= (uint32_t)(y >> 32) | (uint32_t)t;              // t < 0: 2^63 and up
+  return y;
 }
 
 // v 2^-s rounded to nearest even, |v| < 2^63, the result normal.  On the bits:

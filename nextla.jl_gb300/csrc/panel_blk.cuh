@@ -59,7 +59,8 @@ template <int FORM>
 __device__ __forceinline__ unsigned long long v_fixed(const double *P, int ldp, int r, int col, int m, int kcol) {
   double v = (r < m && col < kcol) ? P[(size_t)col * ldp + r] : 0.0;
   if (FORM == 0 && col < kcol) v = r < col ? 0.0 : (r == col ? 1.0 : v);
-  return (unsigned long long)oz::to_fixed<false>(v, 61) + oz::kBias;
+  uint32_t out = 0;                                     // |v| <= 1
+  return oz::to_biased<61>(v, out);
 }
 
 // householder() (common.cuh) for finite alpha and xnorm_sq within the range
