@@ -63,14 +63,16 @@ __device__ __forceinline__ unsigned long long v_fixed(const double *P, int ldp, 
   return oz::to_biased<61>(v, out);
 }
 
-// householder() (common.cuh) for finite alpha and xnorm_sq within the range
-// checks of the block, with the square root and the two divisions as series
-// from FP32 seeds: with y0 ~ v^(-1/2) and r = 1 - v y0^2, v^(-1/2) =
+// householder() (common.cuh) with the square root and the two divisions as
+// series from FP32 seeds: with y0 ~ v^(-1/2) and r = 1 - v y0^2, v^(-1/2) =
 // y0 (1 - r)^(-1/2) = y0 (1 + r/2 + 3 r^2/8 + ...); with z0 ~ 1/d and q = 1 -
 // d z0, 1/d = z0 (1 + q + q^2 + ...).  Seeds are good to 2^-22, so the first
 // terms left out are below 2^-66.  Every FP64 instruction, a comparison or a
 // conversion too, takes its warp 64 clocks whatever depends on it, so what can
 // be done on the bits is: 13 of them here, 25 with the library's operations.
+// The exponent arithmetic is for normal v with room on both sides; a column
+// whose v is outside 2^-959 .. 2^941 (subnormal, infinite and NaN included)
+// goes through householder() itself.  All lanes of the warp have the same one.
 __device__ __forceinline__ bool is_zero(double v) {
   return ((__double2hiint(v) & 0x7fffffff) | __double2loint(v)) == 0;
 }
@@ -82,12 +84,16 @@ __device__ __forceinline__ double from_float(float x) {       // a normal number
   const uint32_t u = __float_as_uint(x);
   return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
 }
+static __device__ __noinline__ bool householder_far(double alpha, double xnorm_sq, double &beta, double &tau, double &scale) {
+  return householder(alpha, xnorm_sq, beta, tau, scale);
+}
 __device__ __forceinline__ bool householder_fast(double alpha, double xnorm_sq, double &beta, double &tau,
                                                  double &scale) {
   if (is_zero(xnorm_sq)) return false;
   const double v = fma(alpha, alpha, xnorm_sq);
   // v = f 4^e with f in [1, 4)
   const int hv = __double2hiint(v), e2 = ((hv >> 20) - 1023) >> 1;
+  if ((uint32_t)(hv >> 20) - 64u > 1900u) return householder_far(alpha, xnorm_sq, beta, tau, scale);
   const double f = __hiloint2double(hv - (e2 << 21), __double2loint(v));
   const double y0 = from_float(rsqrtf(to_float_12(f)));
   const double h = f * y0, r = fma(-h, y0, 1.0);
@@ -177,7 +183,10 @@ __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, i
     // largest s with norm 2^s <= 2^60.9 (oz_apply.cuh)
     const int lg = ((__float_as_int(n2 * (1.0f / 3.48f)) >> 23) & 0xff) - 127;
     if (e == 0) sc2[c] = 60 - ((lg + 2) >> 1) + 1022 - ex;
-    if (!__syncthreads_and(mx == 0 || (ex <= 1900 && ex >= 140))) return false;
+    // the column loop's sums are of products of two entries: between 2^-400
+    // and 2^498 (with the square of 544 rows' norm) none leaves the normal
+    // range, residuals 2^-60 below the column included
+    if (!__syncthreads_and(mx == 0 || (ex <= 1520 && ex >= 623))) return false;
   }
   // ---- the columns right of the first sub-block to fixed point, in place ----
   for (int r = tid; r < m; r += TQR_THREADS)
