@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(TQR_THREADS, OZ ? 1 : 2) k_tree(const TreeGeom
 }
 
 template <typename R>
-static cudaError_t tree_launch(const TreeGeom<R> &g, const TreeOp &op, int ntask, int ny, cudaStream_t st) {
+cudaError_t tree_launch(const TreeGeom<R> &g, const TreeOp &op, int ntask, int ny, cudaStream_t st) {
   if (ntask <= 0 || ny <= 0) return cudaSuccess;
   if constexpr (std::is_same<R, double>::value) {
     if (tree_oz<R>(g.nb, g.ib)) {
@@ -253,7 +253,7 @@ static cudaError_t tree_launch(const TreeGeom<R> &g, const TreeOp &op, int ntask
 }
 
 template <typename R>
-static cudaError_t tree_kernel_attr() {
+cudaError_t tree_kernel_attr() {
   if constexpr (std::is_same<R, double>::value) {
     cudaError_t e = cudaFuncSetAttribute(k_tree<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)oz::kSmem);
     if (e != cudaSuccess) return e;
@@ -1113,7 +1113,7 @@ static size_t tree_work_bytes(TreeShape sh) {
 }
 
 template <typename R, bool TC, bool OZ = false, bool F64P = false>
-static cudaError_t tree_dag_launch(const TDagArgs<R> &a, size_t sm, cudaStream_t st) {
+cudaError_t tree_dag_launch(const TDagArgs<R> &a, size_t sm, cudaStream_t st) {
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(k_tree_dag<R, TC, OZ, F64P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) !=
       cudaSuccess)
@@ -1130,6 +1130,23 @@ static cudaError_t tree_dag_launch(const TDagArgs<R> &a, size_t sm, cudaStream_t
   count_launch();
   return cudaGetLastError();
 }
+
+// The FP32 kernels are a translation unit of their own (tree_f32.cu, this file
+// up to here): in one the two halves take minutes longer to compile.
+#ifdef TREE_F32
+#define TREE_F32_INST template
+#else
+#define TREE_F32_INST extern template
+#endif
+TREE_F32_INST cudaError_t tree_launch<float>(const TreeGeom<float> &, const TreeOp &, int, int, cudaStream_t);
+TREE_F32_INST cudaError_t tree_kernel_attr<float>();
+TREE_F32_INST cudaError_t tree_dag_launch<float, false>(const TDagArgs<float> &, size_t, cudaStream_t);
+TREE_F32_INST cudaError_t tree_dag_launch<float, true>(const TDagArgs<float> &, size_t, cudaStream_t);
+TREE_F32_INST cudaError_t tree_dag_launch<float, false, false, true>(const TDagArgs<float> &, size_t, cudaStream_t);
+TREE_F32_INST cudaError_t tree_dag_launch<float, true, false, true>(const TDagArgs<float> &, size_t, cudaStream_t);
+#ifdef TREE_F32
+}  // namespace tqr
+#else
 
 // mixed: FP32 only -- FP64 panel steps (and tensor-core updates where the
 // shape allows), the factorisation of the mixed-precision solve.  Plain FP32
@@ -1497,3 +1514,4 @@ int tqr_stile_geqrf_tree_dag(int m, int n, int nb, int ib, float *A, int lda, fl
 }
 
 }  // extern "C"
+#endif  // TREE_F32

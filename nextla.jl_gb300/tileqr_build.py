@@ -17,7 +17,11 @@ LIB = os.path.join(OUT_DIR, "libtileqr.so")
 OBJ_DIR = os.path.join(HERE, "_build")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVFLAGS = ["-O3", "--split-compile=0", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
+NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
+# Splitting a file's device code over threads changes its register allocation, mostly for the worse: FP32
+# 256-row tsmqr 150 us against 144, 64-row FP32 tile step 554 against 480, 8192^2 FP64 174 ms against 167.  The FP32
+# tree kernels come out better (32768 x 4096 mixed least squares 96.9 ms against 99.2), and are the longest to compile.
+SPLIT = {"tree_f32.cu"}
 
 
 def nvcc():
@@ -51,7 +55,8 @@ def build(force=False, verbose=False):
 
     def compile_one(src):
         obj = os.path.join(OBJ_DIR, os.path.basename(src)[:-3] + ".o")
-        cmd = [nv, *ARCH, *NVFLAGS, "-I", CSRC, "-I", INCLUDE, "-c", src, "-o", obj]
+        split = ["--split-compile=0"] if os.path.basename(src) in SPLIT else []
+        cmd = [nv, *ARCH, *NVFLAGS, *split, "-I", CSRC, "-I", INCLUDE, "-c", src, "-o", obj]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed on {src}:\n{r.stdout}\n{r.stderr}")
