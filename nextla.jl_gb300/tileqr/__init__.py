@@ -437,13 +437,18 @@ def _tile_geqrf_padded(A, nb, ib, T, tau):
     """Tile QR of a matrix that is not whole tiles on the persistent kernel:
     the matrix extended by zero rows and columns, which no reflector touches
     and which add no reflector of their own, and only what the call writes
-    copied back.  The stream driver, which takes any shape, runs one panel
+    copied back.  (A column of one row has no reflector, but a complex one of
+    nonzero imaginary part gets one as soon as zero rows follow it; only a
+    matrix with a last tile row short of rows and no more rows than columns
+    ends in such a column, and stays with the stream driver.)  That driver, which takes any shape, runs one panel
     kernel after another on one SM: 2900 x 1500 FP64 in 63 ms against 12 ms.
     Returns False (nothing done) where the persistent kernel does not apply."""
     import ctypes
     m, n = A.shape
     if nb <= 0 or ib <= 0 or A.dtype == torch.float32 or torch.cuda.is_current_stream_capturing():
         return False                       # FP32: its tensor-core updates round differently
+    if A.dtype.is_complex and m <= n and m % nb:
+        return False
     mp, np_ = -(-m // nb) * nb, -(-n // nb) * nb
     size = dag_worksize(mp, np_, nb, ib)
     if size is None or min(m, n) <= 0 or mp + np_ <= 2 * nb:
