@@ -152,15 +152,17 @@ template <typename R, int NW, int VEC = 0>
 __device__ bool apply_strip(const ApplyArgs<R> &a, int c0, unsigned char *smem_raw)
 {
   const int tid = threadIdx.x;
-  const int nwl = min(NW, a.ncols - c0);
+  int nwl = min(NW, a.ncols - c0);
   if (nwl <= 0) return false;
   if constexpr (VEC != 0 && std::is_same<R, double>::value && NW <= oz::kCols) {
-    if (oz::covers(a.mode, a.L, a.k, a.ib)) {
-      if (a.L <= 256) {
-        if (oz::strip<1>(a, c0, nwl, smem_raw, a.reuse != 0)) return a.k <= a.ib;
-      } else if constexpr (VEC == 2) {
-        if (oz::strip<2>(a, c0, nwl, smem_raw, false)) return false;
-      }
+    if (oz::covers(a.mode, a.L, a.k, a.ib) && (a.L <= 256 || VEC == 2)) {
+      int fail = 0;
+      if (a.L <= 256) fail = oz::strip<1>(a, c0, nwl, smem_raw, a.reuse != 0);
+      else if constexpr (VEC == 2) fail = oz::strip<2>(a, c0, nwl, smem_raw, false);
+      if (fail == 0) return a.L <= 256 && a.k <= a.ib;
+      // the loops below for the columns of the groups handed back
+      if (fail == 1) nwl = min(nwl, 8);
+      if (fail == 2) { c0 += 8; nwl -= 8; }
     }
   }
   const int L = a.L, ib = a.ib;

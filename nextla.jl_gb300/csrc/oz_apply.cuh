@@ -115,11 +115,16 @@ __device__ __forceinline__ void load_v(const ApplyArgs<double> &a, const double 
 }
 
 // Applies to the strip of columns [c0, c0 + nwl), nwl <= 16, over at most 256
-// J rows.  reuse: V and T are those of the strip just done (true returned, one
-// block, J = 1), their digits still in place.  False: the strip needs the DFMA
-// path; nothing has been written.  All threads get the same answer.
+// J rows.  reuse: V and T are those of the strip just done (0 returned, one
+// block, J = 1), their digits still in place.  Returns which groups of eight
+// columns (bit u: columns 8 u .. 8 u + 7) need the DFMA path; nothing of those
+// has been written.  All threads get the same answer.
+//
+// Whatever depends on the columns' values is decided for such a group alone:
+// strips are 8 or 16 columns wide and start at multiples of 8 in every driver,
+// so a column's bits do not depend on the strip it is in.
 template <int J>
-__device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem, bool reuse) {
+__device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, unsigned char *smem, bool reuse) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int L = a.L, ib = a.ib, k = a.k;
   unsigned char *const Vd = smem + (size_t)warp * kWarpV, *const Td = smem + kOffT, *const Wd = smem + kOffW;
@@ -130,8 +135,8 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
   long long *const A1s = reinterpret_cast<long long *>(smem + kOffA1);
   const bool tt = a.mode == 1 && a.tt >= 0;
   const int Lt = tt ? min(L, a.tt + k) : L;            // rows any reflector touches
-  int bad = 0;
-  uint32_t big = 0, vout = 0;                          // vout: top bit set by a V or T out of range
+  int bad = 0;                                         // bit u: group u
+  uint32_t big[2] = {0, 0}, vout = 0;                  // vout: top bit set by a V or T out of range
 
   // ---- the strip, and A1's rows, from global memory ----
   double *const Cg = a.C + (size_t)c0 * a.c_cs;
@@ -206,7 +211,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
 #pragma unroll
     for (int w = 0; w < 9; ++w) m = max(m, red[w * kCols + c]);
     const int e = m ? (int)(m >> 20) : 1023;           // any scale will do for a column of zeros
-    bad |= (m != 0) & ((e > 1900) | (e < 140));        // far from the ends of the range only
+    bad |= ((m != 0) & ((e > 1900) | (e < 140))) << (c >> 3);   // far from the ends of the range only
     return e;
   };
   const int e0 = col_exp(g), e1 = col_exp(g + 8), ea = col_exp(ca);
@@ -329,20 +334,23 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
     }
     // ---- this warp's share of V^T C, 16 reflectors x 8 columns at a time ----
     // a column's norm leaves its elements a few bits below the digits' range:
-    // 4 C instead of C where no element of the warp reaches 2^59
-    uint32_t far = 0;
+    // 4 C instead of C where no element of the warp and group reaches 2^59
+    uint32_t mul[2];
+    unsigned long long off4[2];                         // biased values: 4 (y - bias) + bias
 #pragma unroll
-    for (int ch = 0; ch < J; ++ch)
+    for (int u = 0; u < 2; ++u) {
+      uint32_t far = 0;
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
+      for (int ch = 0; ch < J; ++ch)
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
           for (int e = 0; e < 2; ++e) far |= (uint32_t)(X[ch][u][q][e] >> 32) - (uint32_t)(kBias >> 32) + 0x08000000u;
-    const bool up = __all_sync(0xffffffffu, far < 0x10000000u);
-    const uint32_t mul = up ? 4u : 1u;
-    const unsigned long long off4 = up ? 0ull - 3ull * kBias : 0ull;       // biased values: 4 (y - bias) + bias
-    if (lane == 0) shw[warp] = up ? 2u : 0u;
+      const bool up = __all_sync(0xffffffffu, far < 0x10000000u);
+      mul[u] = up ? 4u : 1u;
+      off4[u] = up ? 0ull - 3ull * kBias : 0ull;
+      if (lane == 0) shw[2 * warp + u] = up ? 2u : 0u;
+    }
     bool any = false;                                   // this warp's share has been started
 #pragma unroll
     for (int ch = 0; ch < J; ++ch) {
@@ -357,7 +365,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const unsigned long long v = (unsigned long long)X[ch][u][q][e];
-            y[e] = (unsigned long long)(uint32_t)v * mul + off4 + ((unsigned long long)((uint32_t)(v >> 32) * mul) << 32);
+            y[e] = (unsigned long long)(uint32_t)v * mul[u] + off4[u] + ((unsigned long long)((uint32_t)(v >> 32) * mul[u]) << 32);
           }
           digits(y[0], y[1], [&](int d, uint32_t w) { cd[d][q] = w; });
         }
@@ -377,14 +385,14 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
                 mma(acc[d + j], av[0], av[1], av[2], av[3], cd[j][2 * kt], cd[j][2 * kt + 1]);
             }
           long long *wp = Wp + ((size_t)warp * kCols + 8 * u + 2 * t) * kLdWp + 16 * mt + g;
-          const long long z0 = recon<47>(acc, 0, big), z1 = recon<47>(acc, 1, big);
-          const long long z2 = recon<47>(acc, 2, big), z3 = recon<47>(acc, 3, big);
+          const long long z0 = recon<47>(acc, 0, big[u]), z1 = recon<47>(acc, 1, big[u]);
+          const long long z2 = recon<47>(acc, 2, big[u]), z3 = recon<47>(acc, 3, big[u]);
           if (J == 1 || !any) {
             wp[0] = z0; wp[kLdWp] = z1; wp[8] = z2; wp[kLdWp + 8] = z3;
           } else {
             // two shares below 1.25 * 2^62 each: the sum's range is checked on the halves
             bad |= (int)(((uint64_t)((wp[0] >> 1) + (z0 >> 1) + (1ll << 62)) | (uint64_t)((wp[kLdWp] >> 1) + (z1 >> 1) + (1ll << 62)) |
-                          (uint64_t)((wp[8] >> 1) + (z2 >> 1) + (1ll << 62)) | (uint64_t)((wp[kLdWp + 8] >> 1) + (z3 >> 1) + (1ll << 62))) >> 63);
+                          (uint64_t)((wp[8] >> 1) + (z2 >> 1) + (1ll << 62)) | (uint64_t)((wp[kLdWp + 8] >> 1) + (z3 >> 1) + (1ll << 62))) >> 63) << u;
             wp[0] += z0; wp[kLdWp] += z1; wp[8] += z2; wp[kLdWp + 8] += z3;
           }
         }
@@ -406,12 +414,12 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         const int wlo = J == 1 ? r0 >> 5 : 0, whi = J == 1 ? (Lr + 31) >> 5 : 8;
         for (int ww = wlo; ww < whi; ++ww) {
           if (J > 1 && !active(0, ww) && !active(1, ww)) continue;
-          const uint32_t sh = shw[ww];
+          const uint32_t sh = shw[2 * ww + u];
           const long long v = (Wp[((size_t)ww * kCols + c) * kLdWp + q] + (long long)sh) >> sh;   // rounded
           w += v;
           top += (int)(v >> 36);
         }
-        bad |= (top > (1 << 26) - (1 << 18)) | (top < -(1 << 26) + (1 << 18));     // |w| < 0.996 * 2^62
+        bad |= ((top > (1 << 26) - (1 << 18)) | (top < -(1 << 26) + (1 << 18))) << u;   // |w| < 0.996 * 2^62
       }
       W1[c * kLdW1 + q] = w + (long long)kBias;
     }
@@ -439,7 +447,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         const int c = g + 8 * u, p = 8 * warp + 2 * t;
-        const long long w0 = recon<48>(acc, 2 * u, big), w1 = recon<48>(acc, 2 * u + 1, big);
+        const long long w0 = recon<48>(acc, 2 * u, big[u]), w1 = recon<48>(acc, 2 * u + 1, big[u]);
         if (a.mode == 1 && c < nwl) {
           long long *ap = A1s + c * kKMax + i + p;
           if (p < kb) ap[0] -= w0;
@@ -447,7 +455,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         }
         const uint32_t off = plane_off(c, p);
         const unsigned long long y0 = (unsigned long long)w0 + kBias, y1 = (unsigned long long)w1 + kBias;
-        bad |= (int)((uint32_t)((y0 | y1) >> 32) >> 31);              // outside the digits' range
+        bad |= (int)((uint32_t)((y0 | y1) >> 32) >> 31) << u;         // outside the digits' range
         digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Wd + d * kPlaneW + off) = w; });
       }
     }
@@ -479,16 +487,19 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
         for (int u = 0; u < 2; ++u)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const long long dx = recon<47>(acc, 2 * u + e, big);
+            const long long dx = recon<47>(acc, 2 * u + e, big[u]);
             if (J == 1 && dx != 0) changed |= 1u << (8 * u + 2 * q + e);
             X[ch][u][q][e] -= dx;
-            bad |= (int)((uint32_t)(X[ch][u][q][e] >> 32) >> 31);   // left the biased range
+            bad |= (int)((uint32_t)(X[ch][u][q][e] >> 32) >> 31) << u;   // left the biased range
           }
       }
       __syncwarp();
     }
   }
-  if (__syncthreads_or(bad | (int)((big & kBig) != 0) | (int)(vout >> 31))) return false;
+  bad |= (int)((big[0] & kBig) != 0) | (int)((big[1] & kBig) != 0) << 1 | (vout >> 31 ? 3 : 0);
+  const int all = nwl > 8 ? 3 : 1;                      // the strip's groups
+  const int fail = ((__syncthreads_or(bad & 1) ? 1 : 0) | (__syncthreads_or(bad & 2) ? 2 : 0)) & all;
+  if (fail == all) return fail;
 
   // ---- back to FP64: the elements whose value changed ----
 #pragma unroll
@@ -506,7 +517,7 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const long long v = X[ch][u][q][e] - (long long)kBias;
-          moved[e] = c < nwl && r + e < Lt &&
+          moved[e] = c < nwl && r + e < Lt && !((fail >> u) & 1) &&
                      (J == 1 ? ((changed >> (8 * u + 2 * q + e)) & 1u) != 0 : v != to_fixed<true>(x[ch][u][q][e], s));
           y[e] = from_fixed(v, s);
         }
@@ -519,14 +530,14 @@ __device__ __noinline__ bool strip(const ApplyArgs<double> &a, int c0, int nwl, 
       }
   }
 #pragma unroll 8
-  for (int r = la; r < ka; r += 16) {
+  for (int r = la; r < ((fail >> (ca >> 3)) & 1 ? 0 : ka); r += 16) {
     double *pe = A1g + (size_t)r * a.a_rs;
     const double o = __ldcg(pe);
     const long long v = A1s[ca * kKMax + r];
     if (v != to_fixed<true>(o, sa)) *pe = from_fixed(v, sa);
   }
   __syncthreads();
-  return true;
+  return fail;
 }
 
 }  // namespace oz
