@@ -26,7 +26,21 @@
 // the fixed point is 2^-61 sqrt(r) c; the dropped digit products (i + j > 6)
 // add about 2^2 units to W and to C, where the FP64 sums they replace round
 // 256 and 32 times at 2^-53.  Against extended precision a 256-row tsmqr is
-// 3.0e-16 off, normwise, with the FP64 loops 4.4e-16.
+// 1.7e-16 off, normwise, with the FP64 loops 4.4e-16.
+//
+// That is by the column's norm (2^-58.7 of it, 256 rows); the FP64 loops round
+// element i by its own size and that of sum_p |v_ip| |w_p|, which for a row
+// much lighter than the others is far less.  So a group of eight columns goes
+// to those loops if a row some block moved was light in all of them: neither
+// the element, before or after, nor that sum at any block (by the highest
+// digits: one more mma in 28) reached 2^-8.4 of the norm.  Rows of A1 take W itself; they and W are
+// light below 2^-12.4 (A1 is the part above: rows lighter than those of C
+// below it have no accuracy of their own to lose, which |V|^T |C| tells).
+// Elements below 2^-40, but not zero, of [A1; C] or V are handed back at once.
+// Root mean square row error, in roundings of the row's own size, split / FP64
+// loops (k = 32, lower half of 256 rows scaled): equal rows 0.39 / 0.86, 2^-2
+// 0.56 / 1.01, 2^-4 2.0 / 1.1; 2^-6 and lighter is handed back.  Cost: 8192^2
+// 2.5 %.  A column that loses or gains a neighbour outside its group keeps its bits.
 //
 // Layout.  Warp w owns rows [32 w, 32 w + 32) of the strip in registers, as
 // the accumulator fragment of (V W)^T: lane (g, t) = (lane / 4, lane % 4)
@@ -59,14 +73,19 @@ constexpr uint32_t kPlaneV = 32 * 64;  // one digit plane of 32 rows of V: 32 re
 constexpr uint32_t kWarpV = kD * kPlaneV;
 constexpr uint32_t kPlaneW = 16 * 64;
 constexpr int kLdWp = 36, kLdW1 = 40;
-// shared memory: V digits | T digits | W digits | W | partial W | reductions | A1
+// Light or heavy (Accuracy): elements by the high word of their fixed point,
+// sums of |v| |w| in units of the highest digits (2^-7, 2^54).  Rows of C:
+// 2^-8.4 of the column's norm; W and A1: 2^-12.4.
+constexpr uint32_t kHeavy = 3u << 18, kHeavyW = 3u << 14;
+constexpr float kHeavySum = 24.0f, kHeavySumW = 1.0f;
+// shared memory: V digits | T digits | W digits | W | partial W | reductions | flags | A1
 constexpr size_t kOffT = 8 * (size_t)kWarpV;
 constexpr size_t kOffW = kOffT + kD * (size_t)kPlaneV;
-constexpr size_t kOffW1 = kOffW + kD * (size_t)kPlaneW;
+constexpr size_t kOffW1 = kOffW + (kD + 1) * (size_t)kPlaneW;   // and |W| by its highest digits
 constexpr size_t kOffWp = kOffW1 + sizeof(long long) * kCols * kLdW1;
 constexpr size_t kOffRed = kOffWp + sizeof(long long) * 8 * kCols * kLdWp;
 constexpr size_t kOffSh = kOffRed + sizeof(uint32_t) * kCols * 9;
-constexpr size_t kOffA1 = kOffSh + sizeof(uint32_t) * 16;
+constexpr size_t kOffA1 = kOffSh + sizeof(uint32_t) * 32;
 constexpr size_t kSmem = kOffA1 + sizeof(long long) * kCols * kKMax;
 static_assert(kSmem <= TQR_SMEM_MAX, "one CTA's shared memory");
 
@@ -131,7 +150,10 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
   long long *const W1 = reinterpret_cast<long long *>(smem + kOffW1);
   long long *const Wp = reinterpret_cast<long long *>(smem + kOffWp);
   uint32_t *const red = reinterpret_cast<uint32_t *>(smem + kOffRed);   // [warp 0..7, A1][column]
-  uint32_t *const shw = reinterpret_cast<uint32_t *>(smem + kOffSh);    // per warp: V^T C's share is scaled by 2^shw
+  uint32_t *const shw = reinterpret_cast<uint32_t *>(smem + kOffSh);    // per warp and group: V^T C's share is scaled by 2^shw
+  uint32_t *const light = shw + 16;                    // [block parity][group]: reflectors whose W is light
+  uint32_t *const heavy = shw + 20;                    // [group]: those of them whose |V|^T |C| is not
+  if (tid < 16) light[tid] = 0;
   long long *const A1s = reinterpret_cast<long long *>(smem + kOffA1);
   const bool tt = a.mode == 1 && a.tt >= 0;
   const int Lt = tt ? min(L, a.tt + k) : L;            // rows any reflector touches
@@ -176,12 +198,13 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
   double *const A1g = a.mode == 1 ? a.A1 + (size_t)(c0 + ca) * a.a_cs : nullptr;
   const int ka = a.mode == 1 && ca < nwl ? k : 0;
   double *const A1c = reinterpret_cast<double *>(A1s) + ca * kKMax;
-  uint32_t m0 = 0, m1 = 0, ma = 0;
+  uint32_t m0 = 0, m1 = 0, ma = 0, l0 = ~0u, l1 = ~0u, lo = ~0u;   // largest; smallest but zero, less one, in this lane
 #pragma unroll 8
   for (int r = la; r < ka; r += 16) {
     const double v = __ldcg(A1g + (size_t)r * a.a_rs);
     A1c[r] = v;
     ma = max(ma, mag(v));
+    lo = min(lo, mag(v) - 1u);
   }
   // ---- column scales: largest exponent, then the norm ----
 #pragma unroll
@@ -192,6 +215,8 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
       for (int e = 0; e < 2; ++e) {
         m0 = max(m0, mag(x[ch][0][q][e]));
         m1 = max(m1, mag(x[ch][1][q][e]));
+        l0 = min(l0, mag(x[ch][0][q][e]) - 1u);
+        l1 = min(l1, mag(x[ch][1][q][e]) - 1u);
       }
 #pragma unroll
   for (int o = 1; o <= 2; o <<= 1) {
@@ -260,16 +285,26 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
   };
   const int s0 = col_scale(g, e0), s1 = col_scale(g + 8, e1), sa = col_scale(ca, ea);
   long long X[J][2][4][2];                             // biased by kBias
-  uint32_t changed = 0;                                // J = 1: elements some block moved
+  uint32_t row[J];                                     // bit 8 u + 2 q + e: heavy element; + 16: element some block moved
+  auto high = [](long long v) { return (uint32_t)abs((int)(uint32_t)(v >> 32)); };
+  // high word of an FP64 magnitude of 1.5 * 2^e in fixed point
+  auto level = [](int e, int s) { return ((uint32_t)(1023 + e - s) << 20) + 0x80000u; };
+  // elements below 2^-40 of the norm, but not zero
+  bad |= (int)(l0 < level(20, s0)) | (int)(l1 < level(20, s1)) << 1 | (int)(lo < level(20, sa)) << (ca >> 3);
+  const uint32_t t0 = level(51, s0), t1 = level(51, s1);        // kHeavy
 #pragma unroll
-  for (int ch = 0; ch < J; ++ch)
+  for (int ch = 0; ch < J; ++ch) {
+    row[ch] = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        X[ch][0][q][e] = to_fixed<true>(x[ch][0][q][e], s0) + (long long)kBias;
-        X[ch][1][q][e] = to_fixed<true>(x[ch][1][q][e], s1) + (long long)kBias;
-      }
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (mag(x[ch][u][q][e]) >= (u ? t1 : t0)) row[ch] |= 1u << (8 * u + 2 * q + e);
+          X[ch][u][q][e] = to_fixed<true>(x[ch][u][q][e], u ? s1 : s0) + (long long)kBias;
+        }
+  }
 #pragma unroll 2
   for (int r = la; r < ka; r += 16) A1s[ca * kKMax + r] = to_fixed<true>(A1c[r], sa);
 
@@ -303,6 +338,7 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
                           (a.mode == 0 ? rw >= i + kb : !tt || rw + 32 <= a.tt + i + 1);
       constexpr int kStep = 8;                         // reflectors of a pass
       int p = lane >> 4;
+      uint32_t least = ~0u;
       double v[4][2], n[4][2];
       load_v(a, Vg, wholev, r, p, kb, i, Lr, tt, v);
 #pragma unroll 1
@@ -312,12 +348,15 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
         for (int u = 0; u < 4; ++u) {
           const unsigned long long y0 = to_biased<61>(v[u][0], vout);
           const unsigned long long y1 = to_biased<61>(v[u][1], vout);
+          least = min(least, ((uint32_t)__double2hiint(v[u][0]) & 0x7fffffffu) - 1u);
+          least = min(least, ((uint32_t)__double2hiint(v[u][1]) & 0x7fffffffu) - 1u);
           const uint32_t off = plane_off(p + 2 * u, 2 * (lane & 15));
           digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Vd + d * kPlaneV + off) = w; });
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) { v[u][0] = n[u][0]; v[u][1] = n[u][1]; }
       }
+      if (least < (1023u - 40u) << 20) vout |= 0x80000000u;       // an entry of V below 2^-40, but not zero
       __syncwarp();
     };
     if (!reuse && active(0, warp)) v_chunk(0);
@@ -401,6 +440,10 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
     }
     __syncthreads();
     // ---- W1 = A1 rows + the warps' shares ----
+    if (tid < 2) {
+      light[2 * ((b + 1) & 1) + tid] = 0;               // last read in the block before
+      heavy[tid] = 0;
+    }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int q = tid & 31, c = (tid >> 5) + 8 * u;
@@ -448,18 +491,74 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
       for (int u = 0; u < 2; ++u) {
         const int c = g + 8 * u, p = 8 * warp + 2 * t;
         const long long w0 = recon<48>(acc, 2 * u, big[u]), w1 = recon<48>(acc, 2 * u + 1, big[u]);
+        const longlong2 wv = *reinterpret_cast<const longlong2 *>(W1 + c * kLdW1 + p);
+        uint32_t hn = 0;                                // bits 0, 1: W before or after T or A1's row heavy; 2, 3: not zero
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const long long v = (e ? wv.y : wv.x) - (long long)kBias, w2 = e ? w1 : w0;
+          hn |= (uint32_t)(max(high(v), high(w2)) >= kHeavyW) << e | (uint32_t)(v != 0 || w2 != 0) << (e + 2);
+        }
         if (a.mode == 1 && c < nwl) {
           long long *ap = A1s + c * kKMax + i + p;
-          if (p < kb) ap[0] -= w0;
-          if (p + 1 < kb) ap[1] -= w1;
+          if (p < kb) {
+            hn |= (uint32_t)(high(ap[0]) >= kHeavyW);
+            ap[0] -= w0;
+          }
+          if (p + 1 < kb) {
+            hn |= (uint32_t)(high(ap[1]) >= kHeavyW) << 1;
+            ap[1] -= w1;
+          }
         }
+#pragma unroll
+        for (int o = 4; o <= 16; o <<= 1) hn |= __shfl_xor_sync(0xffffffffu, hn, o);
+        const uint32_t l = (hn >> 2) & ~hn & 3u;
+        if (g == 0 && l) atomicOr(&light[2 * (b & 1) + u], l << p);
         const uint32_t off = plane_off(c, p);
         const unsigned long long y0 = (unsigned long long)w0 + kBias, y1 = (unsigned long long)w1 + kBias;
         bad |= (int)((uint32_t)((y0 | y1) >> 32) >> 31) << u;         // outside the digits' range
-        digits(y0, y1, [&](int d, uint32_t w) { *reinterpret_cast<uint32_t *>(Wd + d * kPlaneW + off) = w; });
+        digits(y0, y1, [&](int d, uint32_t w) {
+          *reinterpret_cast<uint32_t *>(Wd + d * kPlaneW + off) = w;
+          if (d == 0) *reinterpret_cast<uint32_t *>(Wd + kD * kPlaneW + off) = magnitude(w);
+        });
       }
     }
     __syncthreads();
+    // ---- light W: handed back unless |V|^T |C| over some warp's 32 rows (of the chunk whose digits are in place)
+    // is heavy, which the FP64 loops would have rounded it by ----
+    const uint32_t lw[2] = {light[2 * (b & 1)], light[2 * (b & 1) + 1]};
+    if (lw[0] | lw[1]) {
+      const int ch = J > 1 && active(J - 1, warp) ? J - 1 : 0;
+      if (active(ch, warp)) {
+#pragma unroll 1
+        for (int um = 0; um < 4; ++um) {
+          const int u = um >> 1, p = 16 * (um & 1) + (lane & 15);
+          float am[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+          for (int kt = 0; kt < 2; ++kt) {
+            uint32_t av[4], cm[2];
+            ldsm4(vbase + plane_off(p, 16 * kt + 8 * (lane >> 4)), av);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              unsigned long long y[2];
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                y[e] = (unsigned long long)(J > 1 && ch ? (u ? X[J - 1][1][2 * kt + q][e] : X[J - 1][0][2 * kt + q][e])
+                                                        : (u ? X[0][1][2 * kt + q][e] : X[0][0][2 * kt + q][e]));
+              cm[q] = magnitude(digit<6>(y[0], y[1]));
+            }
+            mma(am, magnitude(av[0]), magnitude(av[1]), magnitude(av[2]), magnitude(av[3]), cm[0], cm[1]);
+          }
+          uint32_t h0 = __ballot_sync(0xffffffffu, fmaxf(am[0], am[1]) >= kHeavySumW);
+          uint32_t h1 = __ballot_sync(0xffffffffu, fmaxf(am[2], am[3]) >= kHeavySumW);
+          uint32_t m = 0;                               // a reflector's four lanes hold two columns each
+#pragma unroll
+          for (int r = 0; r < 8; ++r) m |= (uint32_t)((h0 >> (4 * r) & 15u) != 0) << r | (uint32_t)((h1 >> (4 * r) & 15u) != 0) << (r + 8);
+          if (lane == 0 && m) atomicOr(&heavy[u], m << (16 * (um & 1)));
+        }
+      }
+      __syncthreads();
+      bad |= (int)((lw[0] & ~heavy[0]) != 0) | (int)((lw[1] & ~heavy[1]) != 0) << 1;
+    }
     // ---- C -= V W2 on this warp's rows, 8 rows at a time; the last chunk's digits of V are in place ----
 #pragma unroll
     for (int cj = 0; cj < J; ++cj) {
@@ -468,11 +567,12 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
       if (J > 1 && cj > 0 && active(J - 1, warp)) v_chunk(ch);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        float acc[kD][4];
+        float acc[kD][4], am[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         init_acc(acc);
 #pragma unroll 1
         for (int kt = 0; kt < (two ? 2 : 1); ++kt) {
-          uint32_t wa[kD][4];
+          uint32_t wa[kD][4], wm[4];
+          ldsm4(wbase + kD * kPlaneW + plane_off(lane & 15, 16 * kt + 8 * (lane >> 4)), wm);
 #pragma unroll
           for (int d = 0; d < kD; ++d) ldsm4(wbase + d * kPlaneW + plane_off(lane & 15, 16 * kt + 8 * (lane >> 4)), wa[d]);
 #pragma unroll
@@ -481,6 +581,7 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
             ldsm2t(vbase + d * kPlaneV + plane_off(16 * kt + (lane & 15), 8 * q), bv);
 #pragma unroll
             for (int j = 0; j < kD - d; ++j) mma(acc[d + j], wa[j][0], wa[j][1], wa[j][2], wa[j][3], bv[0], bv[1]);
+            if (d == 0) mma(am, wm[0], wm[1], wm[2], wm[3], magnitude(bv[0]), magnitude(bv[1]));
           }
         }
 #pragma unroll
@@ -488,7 +589,8 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const long long dx = recon<47>(acc, 2 * u + e, big[u]);
-            if (J == 1 && dx != 0) changed |= 1u << (8 * u + 2 * q + e);
+            if (dx != 0) row[ch] |= 1u << (16 + 8 * u + 2 * q + e);
+            if (am[2 * u + e] >= kHeavySum) row[ch] |= 1u << (8 * u + 2 * q + e);
             X[ch][u][q][e] -= dx;
             bad |= (int)((uint32_t)(X[ch][u][q][e] >> 32) >> 31) << u;   // left the biased range
           }
@@ -497,6 +599,22 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
     }
   }
   bad |= (int)((big[0] & kBig) != 0) | (int)((big[1] & kBig) != 0) << 1 | (vout >> 31 ? 3 : 0);
+  // rows that moved and were light throughout, in all of the group's columns
+#pragma unroll
+  for (int ch = 0; ch < J; ++ch) {
+    uint32_t r = row[ch];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (high(X[ch][u][q][e] - (long long)kBias) >= kHeavy) r |= 1u << (8 * u + 2 * q + e);
+#pragma unroll
+    for (int o = 4; o <= 16; o <<= 1) r |= __shfl_xor_sync(0xffffffffu, r, o);
+    r = r >> 16 & ~r;
+    bad |= (int)((r & 0xffu) != 0) | (int)((r & 0xff00u) != 0) << 1;
+  }
   const int all = nwl > 8 ? 3 : 1;                      // the strip's groups
   const int fail = ((__syncthreads_or(bad & 1) ? 1 : 0) | (__syncthreads_or(bad & 2) ? 2 : 0)) & all;
   if (fail == all) return fail;
@@ -518,7 +636,7 @@ __device__ __noinline__ int strip(const ApplyArgs<double> &a, int c0, int nwl, u
         for (int e = 0; e < 2; ++e) {
           const long long v = X[ch][u][q][e] - (long long)kBias;
           moved[e] = c < nwl && r + e < Lt && !((fail >> u) & 1) &&
-                     (J == 1 ? ((changed >> (8 * u + 2 * q + e)) & 1u) != 0 : v != to_fixed<true>(x[ch][u][q][e], s));
+                     (J == 1 ? ((row[ch] >> (16 + 8 * u + 2 * q + e)) & 1u) != 0 : v != to_fixed<true>(x[ch][u][q][e], s));
           y[e] = from_fixed(v, s);
         }
         if (vec && moved[0] && moved[1]) {

@@ -96,6 +96,16 @@ __device__ __forceinline__ uint32_t digit(unsigned long long a, unsigned long lo
   return r;
 }
 
+// |digit| of a pair of digits, -1 and 0 both zero: the highest digits of a
+// number then give its magnitude, rounded down.
+__device__ __forceinline__ uint32_t magnitude(uint32_t d) {
+  uint32_t r;
+  asm("add.f16x2 %0, %1, %2;" : "=r"(r) : "r"(d), "r"(0x38003800u));            // + 1/2
+  r &= 0x7fff7fffu;
+  asm("sub.f16x2 %0, %0, %1;" : "+r"(r) : "r"(0x38003800u));
+  return r;
+}
+
 // The seven digits of a pair, highest first, through put(plane, word).
 template <typename F>
 __device__ __forceinline__ void digits(unsigned long long a, unsigned long long b, F &&put) {

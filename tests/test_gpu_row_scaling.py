@@ -1,0 +1,103 @@
+"""FP64 Householder QR of matrices whose rows differ widely in size, heavy rows first: the light rows are
+as accurate, each by its own size, as the heavy ones (the setting of weighted least squares and of equality
+constraints by weighting), through every FP64 path that can use the tensor cores.
+
+Bar: 16 times the error of plain FP64 loops (the oracle) on the same input, row by row against extended
+precision, as heavy and light rows meet in a reflector's sums in an order that is each code's own, plus 32
+sqrt(k) eps of the row's size for k reflectors (a rounding each, at random, and a factor of 32).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+WEIGHTS = [1.0, 1e3, 1e6, 1e12]
+
+
+def F(a):
+    return np.array(a, dtype=np.float64, order="F")
+
+
+def row_scales(m, weight, kind):
+    """heavy: the first eight rows; graded: geometric from 1 down to 1 / weight."""
+    s = np.ones(m)
+    if kind == "heavy":
+        s[:8] = weight
+    else:
+        s = weight ** (-np.arange(m) / max(1, m - 1))
+    return s[:, None]
+
+
+def apply_q(V, T, ib, C, trans, top=None):
+    """Q^T C or Q C in extended precision; top None: V unit lower trapezoidal over C, else [I; V] over [top; C]."""
+    L = np.longdouble
+    C, k = C.astype(L), V.shape[1]
+    top = None if top is None else top.astype(L)
+    blocks = list(range(0, k, ib))
+    for i in (blocks if trans == "C" else blocks[::-1]):
+        kb = min(ib, k - i)
+        Tb = np.triu(T[:kb, i:i + kb]).astype(L)
+        Tb = Tb.T if trans == "C" else Tb
+        if top is None:
+            Vb = np.tril(V[:, i:i + kb].astype(L), -1 - i)
+            Vb[np.arange(i, i + kb), np.arange(kb)] = 1
+            C -= Vb @ (Tb @ (Vb.T @ C))
+        else:
+            Vb = V[:, i:i + kb].astype(L)
+            W = Tb @ (top[i:i + kb] + Vb.T @ C)
+            top[i:i + kb] -= W
+            C -= Vb @ W
+    return C, top
+
+
+def row_error(x, y, size):
+    """Largest error of a row, in units of that row's size."""
+    e = np.max(np.abs((x - y).astype(np.float64)), axis=1)
+    s = np.max(np.abs(np.asarray(size, dtype=np.float64)), axis=1)
+    return float(np.max(e[s > 0] / s[s > 0])) if (s > 0).any() else 0.0
+
+
+def bar(plain, k):
+    return 16 * plain + 32 * np.sqrt(k) * EPS
+
+
+@pytest.mark.parametrize("kind", ["heavy", "graded"])
+@pytest.mark.parametrize("weight", WEIGHTS)
+@pytest.mark.parametrize("m,k,ib,w", [(256, 32, 32, 16), (192, 96, 32, 24), (256, 256, 32, 8), (130, 64, 16, 9)])
+def test_tsmqr_rows(tq, oracle, kind, weight, m, k, ib, w):
+    """[R; A2] with R's rows (the first) heavy and A2's light, and columns scaled alike."""
+    rng = np.random.default_rng(m + k)
+    s = row_scales(k + m, weight, kind)
+    R, V = F(np.triu(rng.standard_normal((k, k)) * s[:k])), F(rng.standard_normal((m, k)) * s[k:])
+    T, tau = np.zeros((ib, k), order="F"), np.zeros(k)
+    oracle.tsqrt(m, k, ib, R, V, T, tau, np.zeros(ib * k))
+    A1, A2 = F(rng.standard_normal((k, w)) * s[:k]), F(rng.standard_normal((m, w)) * s[k:])
+    for trans in "CN":
+        B1, B2 = tq.to_device(A1), tq.to_device(A2)
+        tq.tsmqr("L", trans, k, w, m, w, k, ib, B1, B2, tq.to_device(V), tq.to_device(T), None)
+        r2, r1 = apply_q(V, T, ib, A2, trans, A1)
+        g, r, a = np.vstack([tq.to_numpy(B1), tq.to_numpy(B2)]), np.vstack([r1, r2]), np.vstack([A1, A2])
+        size = np.hstack([a, r.astype(np.float64)])
+        o1, o2 = A1.copy(order="F"), A2.copy(order="F")
+        oracle.tsmqr("L", trans, k, w, m, w, k, ib, o1, o2, V, T, np.zeros(ib * w))
+        assert row_error(g, r, size) <= bar(row_error(np.vstack([o1, o2]), r, size), k)
+
+
+@pytest.mark.parametrize("kind", ["heavy", "graded"])
+@pytest.mark.parametrize("weight", WEIGHTS)
+@pytest.mark.parametrize("m,k,ib,w", [(256, 64, 32, 20), (256, 256, 32, 8), (400, 64, 32, 16), (160, 33, 16, 5)])
+def test_unmqr_rows(tq, oracle, kind, weight, m, k, ib, w):
+    """Q^T on columns scaled like the factored matrix; Q on the identity, whose zero rows become light ones."""
+    rng = np.random.default_rng(2 * m + k)
+    s = row_scales(m, weight, kind)
+    V, T, tau = F(rng.standard_normal((m, k)) * s), np.zeros((ib, k), order="F"), np.zeros(k)
+    oracle.geqrt(m, k, ib, V, T, tau, np.zeros(ib * k))
+    for trans, C in (("C", F(rng.standard_normal((m, w)) * s)), ("N", F(np.eye(m)[:, :w]))):
+        B = tq.to_device(C)
+        tq.unmqr("L", trans, m, w, k, ib, tq.to_device(V), m, tq.to_device(T), B, None)
+        ref, _ = apply_q(V, T, ib, C, trans)
+        size = np.hstack([C, ref.astype(np.float64)])
+        o = C.copy(order="F")
+        oracle.unmqr("L", trans, m, w, k, ib, V, m, T, o, np.zeros((w, ib), order="F"))
+        assert row_error(tq.to_numpy(B), ref, size) <= bar(row_error(o, ref, size), k)
