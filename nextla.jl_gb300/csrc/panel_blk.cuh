@@ -21,8 +21,14 @@
 // follow the rounding, a second round of barriers.
 //
 // Same result as columns_la_f64 up to rounding; the caller falls back to it
-// when a column's exponents are outside the fixed-point range (returns false
-// before anything is written).
+// (false is returned before anything is written) when a column's exponents are
+// outside the fixed-point range, or a row is light: none of its elements
+// reaches 2^-8 of its column's norm.  The FP64 loops round a row by its own
+// size; the fixed point does by the column's, 2.5e-18 of it (256 rows), which
+// for rows of 2^-8 is 2.2 times as much and grows as they get lighter (a row
+// 2^-12 below forty others: 173 roundings of its own size against 2.2).  With
+// reflectors rounded to FP32 the line is 2^-30.  Elements whose fixed point
+// did not change keep their bits.
 #pragma once
 #include "common.cuh"
 #include "oz_digits.cuh"
@@ -132,11 +138,12 @@ __device__ __forceinline__ void v_digits(const double *P, int ldp, int r0, int c
 }  // namespace blk
 
 // FORM, P, rowb, Ts, tt, round32, zero_t_on_skip and tau as in columns_la_f64
-// (panel_dev.cuh); scr: blk::kScratch bytes of shared memory, 16-byte aligned.
-template <int FORM>
+// (panel_dev.cuh); scr: blk::kScratch bytes of shared memory, 16-byte aligned;
+// orig(r, c): element (r, c) of P as the call found it.
+template <int FORM, typename Orig>
 __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, int rs, double *Ts, int ldts, int m,
                                              int k, int nc, int tt, bool round32, bool zero_t_on_skip, double *tau,
-                                             unsigned char *scr) {
+                                             unsigned char *scr, Orig orig) {
   using namespace blk;
   constexpr int D = oz::kD;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -188,6 +195,21 @@ __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, i
     // range, residuals 2^-60 below the column included
     if (!__syncthreads_and(mx == 0 || (ex <= 1520 && ex >= 623))) return false;
   }
+  // ---- rows much lighter than the columns, a thread a row ----
+  {
+    const int lim = 60 - (round32 ? 30 : 8);
+    bool light = false;
+    for (int r = tid; r < m; r += TQR_THREADS) {
+      int top = -4096;                                  // largest exponent in the columns' scales
+#pragma unroll 8
+      for (int c = 0; c < nc; ++c) {
+        const int h = __double2hiint(P[(size_t)c * ldp + r]) & 0x7fffffff;
+        top = max(top, h ? (h >> 20) - 1023 + sc2[c] : -4096);
+      }
+      light |= top > -4096 && top < lim;
+    }
+    if (__syncthreads_or(light)) return false;
+  }
   // ---- the columns right of the first sub-block to fixed point, in place ----
   for (int r = tid; r < m; r += TQR_THREADS)
     for (int c0 = kW; c0 < nc; c0 += kW) {
@@ -211,13 +233,19 @@ __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, i
     if (j0 > 0)
       for (int r = tid; r < m; r += TQR_THREADS) {
         double *const p = P + (size_t)j0 * ldp + r;
-        double x[kW];
+        double x[kW], o[kW];
 #pragma unroll
         for (int c = 0; c < kW; ++c)
-          if (c < w) x[c] = p[(size_t)c * ldp];
+          if (c < w) {
+            x[c] = p[(size_t)c * ldp];
+            o[c] = orig(r, j0 + c);
+          }
 #pragma unroll
         for (int c = 0; c < kW; ++c)
-          if (c < w) x[c] = oz::from_fixed(__double_as_longlong(x[c]) - (long long)oz::kBias, sc2[j0 + c]);
+          if (c < w) {
+            const long long f = __double_as_longlong(x[c]) - (long long)oz::kBias;
+            x[c] = f == oz::to_fixed<true>(o[c], sc2[j0 + c]) ? o[c] : oz::from_fixed(f, sc2[j0 + c]);
+          }
 #pragma unroll
         for (int c = 0; c < kW; ++c)
           if (c < w) p[(size_t)c * ldp] = x[c];

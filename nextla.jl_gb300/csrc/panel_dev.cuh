@@ -517,7 +517,8 @@ __device__ void panel_qr_cta(int m, int nc, R *A, int lda, R *tau, R *T, int ldt
     // loop (a one-row column, geqr2.jl:32-35, is its empty-norm case)
     if (staged && T && stage_t && nc <= 32) {
       if (VEC && blk::covers(m, nc))
-        done = columns_blk_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, m, k, nc, -1, false, true, tau, sp);
+        done = columns_blk_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, m, k, nc, -1, false, true, tau, sp,
+                                  [=](int r, int cc) { return ldg_cg(A + ix(r, cc, lda)); });
       if (!done)
         columns_la_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, c.d, c.part, c.scal, m, k, nc, -1, false, true,
                           tau);
@@ -638,8 +639,10 @@ __device__ void tsqrt_block_cta(int m, int sb, R *A1, int lda1, R *A2, int lda2,
   if constexpr (std::is_same<R, double>::value) {
     if (staged && sb <= 32) {
       if (VEC && blk::covers(mrow, sb))
-        done = tt >= 0 ? columns_blk_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, false, false, tau, sp)
-                       : columns_blk_f64<1>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, -1, false, false, tau, sp);
+        done = tt >= 0 ? columns_blk_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, false, false, tau, sp,
+                                            [=](int r, int cc) { return r <= tt + cc ? ldg_cg(A2 + ix(r, cc, lda2)) : 0.0; })
+                       : columns_blk_f64<1>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, -1, false, false, tau, sp,
+                                            [=](int r, int cc) { return ldg_cg(A2 + ix(r, cc, lda2)); });
       if (done)
         ;
       else if (tt >= 0)
@@ -720,7 +723,8 @@ __device__ inline void panel_qr_cta_f64(int m, int nc, float *A, int lda, float 
   __syncthreads();
   const int k = min(m, nc);
   if (BLK && blk::covers(m, nc) &&
-      columns_blk_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, m, k, nc, -1, true, true, taus, sp)) {
+      columns_blk_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, m, k, nc, -1, true, true, taus, sp,
+                         [=](int r, int cc) { return (double)ldg_cg(A + ix(r, cc, lda)); })) {
   } else if (nc <= 32) {
     columns_la_f64<0>(c.P, c.ldp, c.P, c.ldp, c.Ts, c.ldts, c.d, c.part, c.scal, m, k, nc, -1, true, true, taus);
   } else {
@@ -855,7 +859,10 @@ __device__ inline void ttqrt_block_cta_f64(int m, int sb, int tt, double *D1, in
   __syncthreads();
   c.rs = ldb;
   if (BLK && blk::covers(mrow, sb) &&
-      columns_blk_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, true, false, taus, sp)) {
+      columns_blk_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, mrow, sb, sb, tt, true, false, taus, sp, [=](int r, int cc) {
+        if (r > tt + cc) return 0.0;
+        return r < tt ? (double)ldg_cg(A2 + ix(r, cc, lda2)) : ldg_cg(D2 + ix(r - tt, cc, ldd2));
+      })) {
   } else if (sb <= 32) {
     columns_la_f64<2>(c.P, c.ldp, B, ldb, c.Ts, c.ldts, c.d, c.part, c.scal, m, sb, sb, tt, true, false, taus);
   } else {
@@ -958,7 +965,8 @@ __device__ inline void tsqrt_block_f64x(int m, int sb, double *D, int ldd, float
     if (lane == 0) part[warp] = s;
   };
   const bool done = BLK && blk::covers(m, sb) &&
-                    columns_blk_f64<1>(P, ldp, B, ldb, Ts, ldts, m, sb, sb, -1, true, false, taus, sp);
+                    columns_blk_f64<1>(P, ldp, B, ldb, Ts, ldts, m, sb, sb, -1, true, false, taus, sp,
+                                       [=](int r, int cc) { return (double)ldg_cg(A2 + ix(r, cc, lda2)); });
   if (!done) {
     norm_partials(0);
     __syncthreads();

@@ -101,3 +101,108 @@ def test_unmqr_rows(tq, oracle, kind, weight, m, k, ib, w):
         o = C.copy(order="F")
         oracle.unmqr("L", trans, m, w, k, ib, V, m, T, o, np.zeros((w, ib), order="F"))
         assert row_error(tq.to_numpy(B), ref, size) <= bar(row_error(o, ref, size), k)
+
+
+def check_factor(A0, A, T, nb, ib):
+    """A0 = Q R row by row, Q from the flat tree's reflectors in extended precision."""
+    m, n = A0.shape
+    k = min(m, n)
+    MT, KT = -(-m // nb), -(-k // nb)
+    rows = [slice(i * nb, min(m, (i + 1) * nb)) for i in range(MT)]
+    X = np.zeros((m, n), dtype=np.longdouble)
+    X[:k] = np.triu(A[:k])
+    for j in reversed(range(KT)):
+        c = slice(j * nb, min(n, (j + 1) * nb))
+        for i in reversed(range(j + 1, MT)):
+            kk = min(rows[j].stop - rows[j].start, c.stop - c.start)
+            X[rows[i]], X[rows[j]] = apply_q(A[rows[i], c][:, :kk], T[i * ib:, c][:, :kk], ib, X[rows[i]], "N", X[rows[j]])
+        kk = min(rows[j].stop - rows[j].start, c.stop - c.start)
+        X[rows[j]], _ = apply_q(A[rows[j], c][:, :kk], T[j * ib:, c][:, :kk], ib, X[rows[j]], "N")
+    return row_error(X, A0, A0)
+
+
+@pytest.mark.parametrize("dag", [True, False])
+@pytest.mark.parametrize("kind", ["heavy", "graded"])
+@pytest.mark.parametrize("weight", [1.0, 1e6, 1e12])
+@pytest.mark.parametrize("m,n,nb,ib", [(256, 128, 128, 32), (512, 64, 256, 32), (300, 100, 256, 16)])
+def test_tile_geqrf_rows(tq, oracle, dag, kind, weight, m, n, nb, ib):
+    rng = np.random.default_rng(m + n)
+    A0 = F(rng.standard_normal((m, n)) * row_scales(m, weight, kind))
+    A = tq.to_device(A0)
+    T, tau = tq.tile_geqrf(A, nb, ib, dag=dag)
+    Ao = A0.copy(order="F")
+    To, _ = oracle.tile_geqrf(Ao, nb, ib)
+    assert check_factor(A0, tq.to_numpy(A), tq.to_numpy(T), nb, ib) <= bar(check_factor(A0, Ao, To, nb, ib), min(m, n))
+
+
+@pytest.mark.parametrize("m,n,ib", [(256, 256, 32), (256, 32, 32), (200, 64, 16), (96, 96, 32)])
+def test_triangular_tiles_keep_their_bits(tq, m, n, ib):
+    """An upper triangular matrix has no reflectors: geqrt returns it as it is, entries far below their
+    column's norm included."""
+    rng = np.random.default_rng(n)
+    A0 = F(np.triu(rng.standard_normal((m, n))))
+    for j in range(0, n, 5):
+        A0[j, j] = 1e-25 * (1 + j)
+    graded = A0 * 2.0 ** -(np.arange(m) / 3.0)[:, None]
+    for X in (A0, F(graded)):
+        A, T, tau = tq.to_device(X), tq.zeros(ib, n), tq.zeros(n, 1)[:, 0]
+        tq.geqrt(m, n, ib, A, T, tau, None)
+        assert np.array_equal(tq.to_numpy(A), X)
+        assert not tau.any()
+
+
+@pytest.mark.parametrize("weight", WEIGHTS)
+def test_weighted_least_squares(tq, oracle, weight):
+    """Consistent weighted systems through the batched solver and the tile solver."""
+    import torch
+    from tileqr import batched as Bt
+    m, n = 400, 64
+    rng = np.random.default_rng(8)
+    A0 = F(rng.standard_normal((m, n)) * row_scales(m, weight, "heavy"))
+    x = rng.standard_normal((n, 2))
+    b = F((A0.astype(np.longdouble) @ x.astype(np.longdouble)).astype(np.float64))
+    plain = max(np.abs(oracle.tile_lstsq(A0[:h].copy(order="F"), b[:h].copy(order="F"), 256, 32) - x).max() for h in (m, 256))
+    bg = Bt.BatchedGels(np.array([m, 256], np.int32), np.array([n, n], np.int32), np.array([2, 2], np.int32),
+                        dtype=torch.float64, tune=False)
+    bg.load([A0, A0[:256]], [b, b[:256]])
+    bg.run()
+    for q in range(2):
+        assert np.abs(bg.x_view(q).cpu().numpy() - x).max() <= bar(plain, n)
+    X = tq.tile_gels(tq.to_device(A0), tq.to_device(b), 256, 32)[0]
+    assert np.abs(tq.to_numpy(X)[:n] - x).max() <= bar(plain, n)
+
+
+@pytest.mark.parametrize("kind", ["heavy", "graded"])
+@pytest.mark.parametrize("weight", WEIGHTS)
+def test_differentiable_qr_rows(tq, oracle, kind, weight):
+    import torch
+    from tileqr import autodiff as AD
+    m, n = 600, 96
+    rng = np.random.default_rng(4)
+    A0 = rng.standard_normal((2, m, n)) * row_scales(m, weight, kind)
+    Q, R = AD.qr(torch.from_numpy(A0).cuda())
+    for p in range(2):
+        QR = Q[p].cpu().numpy().astype(np.longdouble) @ np.triu(R[p].cpu().numpy()).astype(np.longdouble)
+        Qo, Ro, _ = oracle.qr_explicit(A0[p], 256, 32)
+        plain = row_error(Qo.astype(np.longdouble) @ np.triu(Ro).astype(np.longdouble), A0[p], A0[p])
+        assert row_error(QR, A0[p], A0[p]) <= bar(plain, n)
+
+
+@pytest.mark.parametrize("weight", WEIGHTS)
+@pytest.mark.parametrize("grp", [1, 4])
+def test_tree_rows(tq, oracle, weight, grp):
+    """The tree factorisation, through Q^T b and back-substitution."""
+    m, n, nb, ib = 1024, 64, 128, 32
+    rng = np.random.default_rng(6)
+    A0 = F(rng.standard_normal((m, n)) * row_scales(m, weight, "heavy"))
+    x = rng.standard_normal((n, 3))
+    b = F((A0.astype(np.longdouble) @ x.astype(np.longdouble)).astype(np.float64))
+    plain = np.abs(oracle.tile_lstsq(A0.copy(order="F"), b.copy(order="F"), nb, ib) - x).max()
+    B = tq.to_device(b)
+    A = tq.to_device(A0)
+    T, tau, T2, tau2 = tq.tile_geqrf_tree(A, nb, ib, B=B, grp=grp)
+    y = tq.to_numpy(B)[:n].astype(np.longdouble)
+    R = np.triu(tq.to_numpy(A)[:n]).astype(np.longdouble)
+    for r in range(n - 1, -1, -1):
+        y[r] = (y[r] - R[r, r + 1:] @ y[r + 1:]) / R[r, r]
+    assert np.abs(y.astype(np.float64) - x).max() <= bar(plain, n)
