@@ -81,7 +81,8 @@ int geqrt_impl(int m, int n, int ib, R *A, int lda, R *T, int ldt, R *tau, cudaS
     const int sb = ib < k - i ? ib : k - i;
     R *av = A + ix(i, i, lda);
     R *tv = T + ix(0, i, ldt);
-    cudaError_t e = launch_panel_qr<R>(m - i, sb, av, lda, tau + i, tv, ldt, st, cluster);
+    cudaError_t e = launch_panel_qr<R>(m - i, sb, av, lda, tau + i, tv, ldt, st, cluster,
+                                       cluster || fp64_tc_tiles(m, ib));
     if (e != cudaSuccess) return rc(e);
     if (n > i + sb) {
       e = launch_apply<R>(0, 'L', 'C', m - i, n - i - sb, sb, sb, A + ix(i, i + sb, lda), lda,
@@ -236,7 +237,8 @@ int tsqrt_impl(int m, int n, int ib, int m1, R *A1, int lda1, R *A2, int lda2, R
   for (int ii = 0; ii < k; ii += ib) {       // src/tsqrt.jl:146-155
     const int sb = (k - ii) < ib ? (k - ii) : ib;
     cudaError_t e = launch_tsqrt_block<R>(m, sb, A1 + ix(ii, ii, lda1), lda1, A2 + ix(0, ii, lda2),
-                                          lda2, T + ix(0, ii, ldt), ldt, tau + ii, st, -1, cluster);
+                                          lda2, T + ix(0, ii, ldt), ldt, tau + ii, st, -1, cluster,
+                                          cluster || fp64_tc_tiles(m, ib));
     if (e != cudaSuccess) return rc(e);
     if (n > ii + sb) {
       e = launch_apply<R>(1, 'L', 'C', m, n - ii - sb, sb, ib, A2 + ix(0, ii + sb, lda2), lda2,

@@ -807,8 +807,11 @@ static int launch_dag(const DagArgs<R> &a, size_t sm, double flops, cudaStream_t
 
 // Double precision: whether strip updates (oz_apply.cuh) or panel steps
 // (panel_blk.cuh) use the tensor cores, which takes one CTA per SM; what the
-// two do not cover stays on the FP64 loops either way.
-static bool dag_oz(const DagGeom &g) { return oz::covers(1, g.nb, g.nb, g.ib) || blk::covers(g.nb, g.ib); }
+// two do not cover stays on the FP64 loops either way.  Without a tile column
+// right of the panels, the updates are those of single blocks.
+static bool dag_oz(const DagGeom &g) {
+  return fp64_tc_tiles(g.nb, g.ib) && (blk::covers(g.nb, g.ib) || oz::covers(1, g.nb, g.NT > 1 ? g.nb : g.ib, g.ib));
+}
 
 static int launch_dag_oz(const DagArgs<double> &a, size_t sm, double flops, cudaStream_t st, bool timed = true) {
   sm = std::max(sm, oz::kSmem);

@@ -201,7 +201,8 @@ static cudaError_t launch_cluster(const ClusterPanelArgs<E> &a, int mrow, cudaSt
 }
 
 template <typename R>
-cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt, cudaStream_t st, bool cluster) {
+cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt, cudaStream_t st, bool cluster,
+                            bool blk) {
   if (cluster && !blk_panel<R>(m, nc)) {
     ClusterPanelArgs<R> a{0, m, nc, A, lda, nullptr, 1, T, ldt, tau, -1};
     bool used = false;
@@ -214,7 +215,7 @@ cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt,
   if (sm > (size_t)TQR_SMEM_MAX) return cudaErrorInvalidValue;
   auto kern = k_panel_qr<R, false>;
   if constexpr (std::is_same<R, double>::value) {
-    if (staged && stage_t && blk::covers(m, nc)) {
+    if (blk && staged && stage_t && blk::covers(m, nc)) {
       kern = k_panel_qr<R, true>;
       sm += blk::kScratch;
     }
@@ -228,7 +229,7 @@ cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt,
 
 template <typename R>
 cudaError_t launch_tsqrt_block(int m, int sb, R *A1, int lda1, R *A2, int lda2, R *T, int ldt,
-                               R *tau, cudaStream_t st, int tt, bool cluster) {
+                               R *tau, cudaStream_t st, int tt, bool cluster, bool blk) {
   const int mrow = tt >= 0 ? (m < tt + sb ? m : tt + sb) : m;
   if (cluster && !blk_panel<R>(mrow, sb)) {
     ClusterPanelArgs<R> a{1, m, sb, A2, lda2, A1, lda1, T, ldt, tau, tt};
@@ -241,7 +242,7 @@ cudaError_t launch_tsqrt_block(int m, int sb, R *A1, int lda1, R *A2, int lda2, 
   if (sm > (size_t)TQR_SMEM_MAX) return cudaErrorInvalidValue;
   auto kern = k_tsqrt_block<R, false>;
   if constexpr (std::is_same<R, double>::value) {
-    if (staged && blk::covers(mrow, sb)) {
+    if (blk && staged && blk::covers(mrow, sb)) {
       kern = k_tsqrt_block<R, true>;
       sm += blk::kScratch;
     }
@@ -265,16 +266,16 @@ cudaError_t launch_larft(int direct_f, int storev_c, int n, int k, const R *V, i
   return cudaGetLastError();
 }
 
-template cudaError_t launch_panel_qr<double>(int, int, double *, int, double *, double *, int, cudaStream_t, bool);
-template cudaError_t launch_panel_qr<float>(int, int, float *, int, float *, float *, int, cudaStream_t, bool);
-template cudaError_t launch_tsqrt_block<double>(int, int, double *, int, double *, int, double *, int, double *, cudaStream_t, int, bool);
-template cudaError_t launch_tsqrt_block<float>(int, int, float *, int, float *, int, float *, int, float *, cudaStream_t, int, bool);
+template cudaError_t launch_panel_qr<double>(int, int, double *, int, double *, double *, int, cudaStream_t, bool, bool);
+template cudaError_t launch_panel_qr<float>(int, int, float *, int, float *, float *, int, cudaStream_t, bool, bool);
+template cudaError_t launch_tsqrt_block<double>(int, int, double *, int, double *, int, double *, int, double *, cudaStream_t, int, bool, bool);
+template cudaError_t launch_tsqrt_block<float>(int, int, float *, int, float *, int, float *, int, float *, cudaStream_t, int, bool, bool);
 template cudaError_t launch_larft<double>(int, int, int, int, const double *, int, const double *, double *, int, cudaStream_t);
 template cudaError_t launch_larft<float>(int, int, int, int, const float *, int, const float *, float *, int, cudaStream_t);
 
 #define TQR_PANEL_INST(E)                                                                                         \
-  template cudaError_t launch_panel_qr<E>(int, int, E *, int, E *, E *, int, cudaStream_t, bool);                       \
-  template cudaError_t launch_tsqrt_block<E>(int, int, E *, int, E *, int, E *, int, E *, cudaStream_t, int, bool);     \
+  template cudaError_t launch_panel_qr<E>(int, int, E *, int, E *, E *, int, cudaStream_t, bool, bool);                       \
+  template cudaError_t launch_tsqrt_block<E>(int, int, E *, int, E *, int, E *, int, E *, cudaStream_t, int, bool, bool);     \
   template cudaError_t launch_larft<E>(int, int, int, int, const E *, int, const E *, E *, int, cudaStream_t);
 TQR_PANEL_INST(cx<double>)
 TQR_PANEL_INST(cx<float>)

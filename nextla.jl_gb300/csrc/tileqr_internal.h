@@ -11,23 +11,33 @@ bool profiling();
 void *prof_begin(cudaStream_t st);
 void prof_end(void *tok, cudaStream_t st, double flops);
 
+// Whether the tile drivers run FP64 strips and panels on the tensor cores
+// (oz_apply.cuh, panel_blk.cuh), at the price of one CTA per SM: from where a
+// whole tile's strips are covered.  Below, the strips would stay on the FP64
+// loops with half the CTAs for the panels' sake (3072 x 3072, ms, two CTAs
+// against one: nb 64, ib 16 64 and 90, nb 96, ib 16 56 and 68; nb 128, ib 16
+// 54 and 27, nb 64, ib 32 72 and 41).
+inline bool fp64_tc_tiles(int nb, int ib) { return nb * ib >= 64 * 32; }
+
 // geqr2 (+ T when T != nullptr) on an m-by-nc panel: one CTA, or with
 // cluster = true a thread-block cluster splitting the rows when the panel is
-// tall enough (panel_cluster.cuh; different summation order, same bar).
+// tall enough (panel_cluster.cuh; different summation order, same bar).  blk:
+// FP64 panels may take the blocked column loop (panel_blk.cuh).
 template <typename R>
 cudaError_t launch_panel_qr(int m, int nc, R *A, int lda, R *tau, R *T, int ldt, cudaStream_t st,
-                            bool cluster = false);
+                            bool cluster = false, bool blk = true);
 
 // One ib-block of tsqrt (pointers already offset to the block), one CTA or
 // (cluster = true) a cluster; tt >= 0: the ttqrt block whose first column is
 // column tt of the triangle.
 template <typename R>
 cudaError_t launch_tsqrt_block(int m, int sb, R *A1, int lda1, R *A2, int lda2, R *T, int ldt,
-                               R *tau, cudaStream_t st, int tt = -1, bool cluster = false);
+                               R *tau, cudaStream_t st, int tt = -1, bool cluster = false, bool blk = true);
 
 // The C-ABI routines' bodies (capi.cu).  `cluster` selects the cluster panel
 // for the panel steps: the entry points use it; the stream tile driver does
-// not, so that it stays bit-identical to the persistent schedule.
+// not, so that it stays bit-identical to the persistent schedule (and takes
+// the blocked FP64 panels where that does, fp64_tc_tiles).
 template <typename R>
 int geqrt_impl(int m, int n, int ib, R *A, int lda, R *T, int ldt, R *tau, cudaStream_t st, bool cluster);
 template <typename R>

@@ -224,11 +224,15 @@ __device__ void tree_task(const TreeGeom<R> &g, const TreeOp &op, int i, int y, 
   }
 }
 
-// Double precision: whether the strip updates run on the tensor cores
-// (oz_apply.cuh; OZ below), which takes one CTA per SM.
+// Double precision: whether strip updates or panel steps run on the tensor
+// cores (OZ below), which takes one CTA per SM; as dag_oz (dag.cu).  ib = 8 has
+// neither when there is no trailing column (16384 x 256, nb 256: 13.9 ms with
+// two CTAs, 15.1 with one).
 template <typename R>
-static bool tree_oz(int nb, int ib) {
-  return std::is_same<R, double>::value && (oz::covers(1, nb, nb, ib) || blk::covers(nb, ib));
+static bool tree_oz(const TreeGeom<R> &g) {
+  const bool trail = g.n > g.nb || g.nrhs > 0;
+  return std::is_same<R, double>::value && fp64_tc_tiles(g.nb, g.ib) &&
+         (blk::covers(g.nb, g.ib) || oz::covers(1, g.nb, trail ? g.nb : g.ib, g.ib));
 }
 
 template <typename R, bool OZ>
@@ -241,7 +245,7 @@ template <typename R>
 cudaError_t tree_launch(const TreeGeom<R> &g, const TreeOp &op, int ntask, int ny, cudaStream_t st) {
   if (ntask <= 0 || ny <= 0) return cudaSuccess;
   if constexpr (std::is_same<R, double>::value) {
-    if (tree_oz<R>(g.nb, g.ib)) {
+    if (tree_oz<R>(g)) {
       k_tree<R, true><<<dim3(ntask, ny), TQR_THREADS, oz::kSmem, st>>>(g, op);
       count_launch();
       return cudaGetLastError();
@@ -1223,7 +1227,7 @@ static int tree_geqrf_dag_impl(int m, int n, int nb, int ib, R *A, int lda, R *T
     }
   }
   if constexpr (std::is_same<R, double>::value) {
-    if (tree_oz<R>(nb, ib)) {
+    if (tree_oz<R>(a.g)) {
       e = tree_dag_launch<R, false, true>(a, std::max(sm, oz::kSmem), st);
       return e == cudaSuccess ? 0 : (int)e;
     }
