@@ -1302,12 +1302,13 @@ int tqr_tile_dag_occupancy(int dtype_bytes, int tensor_cores, int *ctas_per_sm, 
   cudaError_t e;
   int per = 0;
   if (dtype_bytes == 8) {
+    // the kernel of these tiles (dag_oz)
     sm = std::max({apply_smem_elems(nb, ib, 16, true, true, true) * sizeof(double), panel_smem<double>(nb, ib, true, true),
-                   tsqrt_smem<double>(nb, ib, true)});
-    if ((e = cudaFuncSetAttribute(k_tile_dag<double, 16, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                   tsqrt_smem<double>(nb, ib, true), oz::kSmem});
+    if ((e = cudaFuncSetAttribute(k_tile_dag<double, 16, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sm)) != cudaSuccess)
       return (int)e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<double, 16, false, false>, TQR_THREADS, sm);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tile_dag<double, 16, true, false>, TQR_THREADS, sm);
   } else {
     sm = std::max({apply_smem_elems(nb, ib, 16, true, true, true) * sizeof(float), panel_smem<float>(nb, ib, true, true),
                    tsqrt_smem<float>(nb, ib, true)});
