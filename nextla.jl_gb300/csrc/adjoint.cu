@@ -61,11 +61,16 @@ static size_t adj_smem(bool oz) {
                    apply_smem_elems(256, 32, AdjNW<R>::value, true, true, true) * sizeof(R)});
 }
 
-// Double precision: the trailing updates run on the tensor cores
-// (oz_apply.cuh, one CTA per SM) unless the blocks are too small for them.
+// Double precision: panels and updates run on the tensor cores (panel_blk.cuh,
+// oz_apply.cuh, one CTA per SM) unless the blocks are too small for them, or
+// the problems too narrow to leave them enough (forward and adjoint of 304
+// problems, ms, two CTAs against one: 300 x 24, ib 32 1.58 and 1.59, 300 x 16
+// 0.88 and 0.97, 300 x 12 0.69 and 0.91, 1024 x 12 1.61 and 1.99; 256 of 512 x
+// 32 3.2 and 2.1; ib 8, 300 x 48 4.1 and 4.7, 300 x 64 6.5 and 7.4).
 template <typename R>
 static bool adj_oz(int n, int ib) {
-  return std::is_same<R, double>::value && (oz::covers(1, kAdjNb, n, ib) || blk::covers(kAdjNb, std::min(n, ib)));
+  return std::is_same<R, double>::value && n >= 32 && (ib >= 16 || n >= 128) &&
+         (oz::covers(1, kAdjNb, n, ib) || blk::covers(kAdjNb, std::min(n, ib)));
 }
 
 struct AdjGeom {
