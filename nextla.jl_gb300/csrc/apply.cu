@@ -32,7 +32,10 @@ static cudaError_t launch_oz(ApplyArgs<double> a, cudaStream_t st) {
   count_launch();
   return cudaGetLastError();
 }
-static_assert(sizeof(double) * ((size_t)257 * (oz::kIbMax + oz::kCols) + 3 * 32 * 32) <= oz::kSmem,
+// apply_smem_elems(oz::kRowsMax, oz::kIbMax, oz::kCols, true, true, true)
+static_assert(oz::kIbMax * oz::kCols <= kW2Regs * TQR_THREADS &&
+                  sizeof(double) * ((size_t)(oz::kRowsMax + 1) * (oz::kIbMax + oz::kCols) + oz::kIbMax * oz::kCols +
+                                    oz::kIbMax * oz::kIbMax) <= oz::kSmem,
               "the DFMA path's staged strip fits the same shared memory");
 
 // Fewest CTAs a stand-alone apply should run on before narrower strips are used.
