@@ -433,6 +433,24 @@ def dag_stats():
     return res
 
 
+def _padded_pays(m, n, nb, ib):
+    """Whether a matrix that is not whole tiles is better extended to whole ones.
+    The stream driver takes its panel columns one after another, tile by tile;
+    in the persistent kernel the blocks of a panel's tiles follow one another
+    like a pipeline, padded columns included.  Where the two column counts meet,
+    so do the times (FP64, nb 256, ib 32, ms: 300 x 300 2.5 and 2.6, 257 x 257
+    2.2 and 2.6, 513 x 513 5.7 and 4.1, 4097 x 33 2.9 and 3.3, 4000 x 100 7.8
+    and 3.3; ComplexF64 4097 x 33 13.3 and 13.5, 4000 x 100 37 and 14).  Very
+    narrow matrices would also need many times their memory."""
+    mt, nt = -(-m // nb), -(-n // nb)
+    one_by_one = pipelined = 0
+    for k in range(min(mt, nt)):
+        nk = min(nb, n - k * nb)
+        one_by_one += min(nb, m - k * nb, nk) + (mt - k - 1) * nk
+        pipelined += (mt - k - 1) * ib + nb
+    return one_by_one >= pipelined and mt * nb * nt * nb <= 4 * m * n
+
+
 def _tile_geqrf_padded(A, nb, ib, T, tau):
     """Tile QR of a matrix that is not whole tiles on the persistent kernel:
     the matrix extended by zero rows and columns, which no reflector touches
@@ -450,8 +468,10 @@ def _tile_geqrf_padded(A, nb, ib, T, tau):
     if A.dtype.is_complex and m <= n and m % nb:
         return False
     mp, np_ = -(-m // nb) * nb, -(-n // nb) * nb
+    if min(m, n) <= 0 or mp + np_ <= 2 * nb or not _padded_pays(m, n, nb, ib):
+        return False
     size = dag_worksize(mp, np_, nb, ib)
-    if size is None or min(m, n) <= 0 or mp + np_ <= 2 * nb:
+    if size is None:
         return False
     k = min(m, n)
     try:
