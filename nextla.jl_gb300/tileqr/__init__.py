@@ -401,8 +401,15 @@ def dag_check(m, n, nb, ib):
     return rc, int(nt.value)
 
 
-def dag_status(work_ptr):
+def dag_status(work_ptr=None):
+    """(status, task) of the schedule run in the workspace at work_ptr (by
+    default the last persistent-kernel tile QR's): 0, or why it stopped and at
+    which task; synchronises the current stream."""
     import ctypes
+    if work_ptr is None:
+        if _LAST_DAG_WORK is None:
+            return 0, 0
+        work_ptr = _LAST_DAG_WORK
     s, t = ctypes.c_int(0), ctypes.c_int(0)
     rc = _lib.lib().tqr_tile_dag_status(ctypes.c_void_p(work_ptr), ctypes.byref(s), ctypes.byref(t),
                                         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
@@ -412,6 +419,7 @@ def dag_status(work_ptr):
 
 
 _LAST_DAG_WORK = None
+_LAST_DAG_KEEP = None          # the tensor it lies in, where no cached workspace holds it
 
 DAG_TASKS = ("GB", "GA", "UN", "TB", "TA", "TM")
 
@@ -494,6 +502,8 @@ def _tile_geqrf_padded(A, nb, ib, T, tau):
         return False                       # outside the persistent path for this element type
     if rc > 0:
         raise RuntimeError(f"tile_geqrf: CUDA error {rc}")
+    global _LAST_DAG_WORK, _LAST_DAG_KEEP
+    _LAST_DAG_WORK, _LAST_DAG_KEEP = wp, w
     A.copy_(Ap[:m, :n])
     T[:rows, :k].copy_(Tp[:, :k])
     # the tau of tile (i, j) sits in column i: the tiles above the diagonal have none

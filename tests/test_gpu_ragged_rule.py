@@ -39,3 +39,21 @@ def test_thin_and_barely_ragged_match_the_oracle(tq, oracle, m, n, nb):
     To, tauo = oracle.tile_geqrf(Ao, nb, 32)
     for x, y in ((A, Ao), (T, To), (tau, tauo)):
         assert np.max(np.abs(tq.to_numpy(x) - y)) <= 1e-12 * max(m, n) * np.max(np.abs(y))
+
+
+@pytest.mark.gpu
+def test_status_and_statistics_are_of_the_ragged_call(tq):
+    """Also without blocking, where they are all that tells how the schedule ended."""
+    import torch
+    whole, ragged = (tq.to_device(F(np.random.default_rng(1).standard_normal(s))) for s in ((256, 128), (1000, 700)))
+    tq.tile_geqrf(whole, 128, 32)
+    tq.set_blocking(False)
+    try:
+        small = tq.dag_stats()
+        tq.tile_geqrf(ragged, 128, 32)
+        torch.zeros(64 << 20, device="cuda")            # whatever the call gave back is used again
+        assert tq.dag_status()[0] == 0
+        s = tq.dag_stats()
+    finally:
+        tq.set_blocking(True)
+    assert s["busy_ms_TM"] > 0 and small["busy_ms_TM"] == 0
