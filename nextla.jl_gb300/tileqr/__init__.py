@@ -481,6 +481,8 @@ def _tile_geqrf_padded(A, nb, ib, T, tau):
     size = dag_worksize(mp, np_, nb, ib)
     if size is None:
         return False
+    # memory, as for every other call: no part in an autograd graph
+    A, T, tau = A.data, T.data, tau.data
     k = min(m, n)
     try:
         # scratch of this call only: streams and threads share nothing

@@ -57,3 +57,16 @@ def test_status_and_statistics_are_of_the_ragged_call(tq):
     finally:
         tq.set_blocking(True)
     assert s["busy_ms_TM"] > 0 and small["busy_ms_TM"] == 0
+
+
+@pytest.mark.gpu
+def test_matrices_that_require_gradients(tq):
+    """The factorisation works on the memory of its arguments, in place, like the C entry points."""
+    A0 = F(np.random.default_rng(2).standard_normal((300, 200)))
+    out = []
+    for grad in (False, True):
+        A = tq.to_device(A0).requires_grad_(grad)
+        T, tau = tq.tile_geqrf(A, 128, 32)
+        out.append([tq.to_numpy(x) for x in (A, T, tau)])
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
