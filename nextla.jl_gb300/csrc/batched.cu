@@ -59,7 +59,9 @@ struct BatchHeader {           // first 256 bytes of the workspace
   int bad;                     // descriptors rejected by the kernel
   int first_bad;               // smallest rejected problem index (INT_MAX if none)
   int next_oz;                 // problem counter of the tensor-core pass (double precision)
-  int pad[60];
+  int busy_oz;                 // CTAs working on one of its problems
+  int back;                    // positions its idle CTAs took from the end of the order
+  int pad[58];
 };
 static_assert(sizeof(BatchHeader) == 256, "BatchHeader layout");
 
@@ -86,7 +88,8 @@ __device__ bool update_columns(ApplyArgs<R> a, R *C, int ldc, int ncols, unsigne
 template <typename R, bool OZ>
 __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R *tauscr, unsigned char *smem)
 {
-  const int m = p.m, n = p.n, k = p.k, ib = p.ib;
+  // the descriptor's block size and strip width are the loops' (autotune)
+  const int m = p.m, n = p.n, k = p.k, ib = OZ ? kBatchMaxIb : p.ib;
   R *A = Abase + p.a_off;
   R *B = Bbase + p.b_off;
   const int lda = m, ldb = m;
@@ -101,7 +104,7 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
     a.V = A + ix(i, i, lda); a.ldv = lda;
     a.T = Tscr; a.ldt = ib;
     a.stage_t = 1;
-    const int nw = OZ ? 16 : p.nw;     // the tensor-core strips are 16 columns, whatever the loops prefer
+    const int nw = OZ ? 16 : p.nw;
     constexpr size_t cap = OZ ? oz::kSmem : kBatchSmem;
     const bool full = apply_smem_elems(L, sb, nw, true, true, true) * sizeof(R) <= cap;
     a.stage_v = full;
@@ -144,10 +147,11 @@ __device__ void solve_one(const BatchProblem &p, R *Abase, R *Bbase, R *Tscr, R 
 
 // FP64 problems that a CTA with the SM to itself solves faster, on the
 // tensor-core paths, than two CTAs per SM do on the FP64 loops (2000 equal
-// problems, ms: 256 x 64 5.5 against 7.7, 192 x 150 16.5 against 23.5; 128 x 64
-// 5.05 against 5.01, 128 x 120 13.8 against 12.6, 192 x 32 2.9 against 2.8,
-// 64 x 32 2.8 against 1.7).
-__host__ __device__ inline bool batch_oz(int m, int n) { return m > 128 && n > 32; }
+// problems, ms: 256 x 64 5.3 against 7.7, 192 x 160 17.3 against 24.7, 160 x 64
+// 5.0 against 5.7, 320 x 64 8.1 against 9.3).  Left to the loops: 144 x 128
+// 15.0 against 14.5, 320 x 48 5.86 against 5.97, 160 x 36 3.1 against 2.7; what
+// little there is to gain pays less than the second pass's tail costs.
+__host__ __device__ inline bool batch_oz(int m, int n) { return m >= 160 && n >= 64; }
 
 template <bool OZ> constexpr size_t kBatchDynSmem = OZ ? oz::kSmem : kBatchSmem;
 static_assert(sizeof(double) * ((size_t)513 * 32 + 33 * 32 + TQR_THREADS + 64) + blk::kScratch <= oz::kSmem,
@@ -155,47 +159,88 @@ static_assert(sizeof(double) * ((size_t)513 * 32 + 33 * 32 + TQR_THREADS + 64) +
 
 // One pass over the batch.  Double precision takes two: OZ, the problems of
 // batch_oz; not OZ, the others (every other element type: all of them).  A CTA
-// takes one problem at a time; after one that is not its own it looks at up
-// to 32 at once.
+// takes one problem at a time; after one that is not its own it passes over
+// all that follow and are not, up to 1024 at once.  A CTA that finds no more OZ
+// problems while others still work on theirs starts on the second pass, so
+// that no SMs idle between the two (one after the other, 128 problems of up to
+// 170 rows took 3.1 ms against 2.1 without the first pass): in a large batch
+// from the cheap end of the order, not to be late for the second pass, whose
+// kernel stops where they began.  all: the whole batch in this launch (OZ: both
+// passes).
+constexpr int kLargeBatch = 12;                           // problems per CTA
+constexpr int kPeek = 4;
 template <typename R, bool OZ>
 __global__ void __launch_bounds__(TQR_THREADS, OZ ? 1 : 2)
 k_batched_gels(int nprob, const BatchProblem *__restrict__ probs, const int *__restrict__ order, R *A, R *B,
-               BatchHeader *hdr, R *scratch)
+               BatchHeader *hdr, R *scratch, bool all)
 {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ int s_q;
-  __shared__ unsigned s_mine;
+  __shared__ int s_q, s_id, s_from, s_stop;
   R *Tscr = scratch + (size_t)blockIdx.x * kScrElems;
   R *tauscr = Tscr + kBatchMaxIb * kBatchMaxIb;
-  constexpr bool kSplit = std::is_same<R, double>::value;
-  int *const next = OZ ? &hdr->next_oz : &hdr->next;
-  int take = 1;
+  const bool split = OZ || (std::is_same<R, double>::value && !all);
+  bool oz = OZ;                                           // the pass this CTA is in
+  const bool from_back = OZ && nprob > kLargeBatch * (int)gridDim.x;
+  const int end = OZ ? nprob : nprob - *(volatile int *)&hdr->back;
+  // problem at position q: its index if it is of this pass, else -1
+  auto own = [&](int q) {
+    const int id = order[q];
+    return id >= 0 && id < nprob && problem_ok(probs[id]) && (!split || batch_oz(probs[id].m, probs[id].n) == oz) ? id : -1;
+  };
+  auto reject = [&](int q) {                              // position q is taken: count it if it is no problem
+    const int id = order[q];
+    const bool known = id >= 0 && id < nprob;
+    if (!oz && !(known && problem_ok(probs[id]))) {
+      atomicAdd(&hdr->bad, 1);
+      atomicMin(&hdr->first_bad, known ? id : q);
+    }
+  };
   for (;;) {
-    if (threadIdx.x < 32) {
-      int q0 = 0;
-      if (threadIdx.x == 0) q0 = atomicAdd(next, take);
-      q0 = __shfl_sync(0xffffffffu, q0, 0);
-      const int q = q0 + (int)threadIdx.x;
-      bool mine = false;
-      if ((int)threadIdx.x < take && q < nprob) {
-        const int id = order[q];
-        const bool known = id >= 0 && id < nprob;
-        const bool ok = known && problem_ok(probs[id]);
-        mine = ok && (!kSplit || batch_oz(probs[id].m, probs[id].n) == OZ);
-        if (!ok && !OZ) { atomicAdd(&hdr->bad, 1); atomicMin(&hdr->first_bad, known ? id : q); }
+    int *const next = oz ? &hdr->next_oz : &hdr->next;
+    if (threadIdx.x == 0) {
+      int q = nprob, id = -1;
+      if (!OZ || oz || all) {
+        q = atomicAdd(next, 1);
+      } else if (*(volatile int *)&hdr->busy_oz != 0) {   // else the second pass proper takes over
+        q = from_back ? nprob - 1 - atomicAdd(&hdr->back, 1) : atomicAdd(next, 1);
+        if (q < 0) q = nprob;
       }
-      const unsigned mask = __ballot_sync(0xffffffffu, mine);
-      if (threadIdx.x == 0) { s_q = q0; s_mine = mask; }
+      if (q < end && (id = own(q)) < 0) reject(q);
+      if (OZ && oz && id >= 0) atomicAdd(&hdr->busy_oz, 1);
+      s_q = q;
+      s_id = id;
+      s_from = *(volatile int *)next;
+      s_stop = s_from + kPeek * TQR_THREADS;
     }
     __syncthreads();
-    const int q0 = s_q;
-    unsigned mine = s_mine;
+    const int q = s_q, id = s_id, from = s_from;
+    if (q >= end) {
+      __syncthreads();
+      if (!OZ || !oz) break;
+      oz = false;
+      continue;
+    }
+    if (id < 0 && split && (oz || !from_back)) {
+      for (int w = 0; w < kPeek; ++w) {
+        const int x = from + w * TQR_THREADS + (int)threadIdx.x;
+        if (x >= end || own(x) >= 0) atomicMin(&s_stop, x);
+      }
+      __syncthreads();
+      const int stop = min(s_stop, end);
+      if (threadIdx.x == 0) s_id = stop > from && atomicCAS(next, from, stop) == from ? 0 : -1;
+      __syncthreads();
+      if (s_id == 0)
+        for (int x = from + (int)threadIdx.x; x < stop; x += TQR_THREADS) reject(x);
+    }
     __syncthreads();
-    if (q0 >= nprob) break;
-    take = kSplit && mine == 0 ? min(32, 2 * take) : 1;
-    for (; mine; mine &= mine - 1) {
-      const BatchProblem p = probs[order[q0 + __ffs(mine) - 1]];
-      solve_one<R, OZ>(p, A, B, Tscr, tauscr, smem_raw);
+    if (id < 0) continue;
+    const BatchProblem p = probs[id];
+    if constexpr (OZ) {
+      if (oz) solve_one<R, true>(p, A, B, Tscr, tauscr, smem_raw);
+      else solve_one<R, false>(p, A, B, Tscr, tauscr, smem_raw);
+      if (oz && threadIdx.x == 0) atomicSub(&hdr->busy_oz, 1);
+    } else {
+      solve_one<R, false>(p, A, B, Tscr, tauscr, smem_raw);
     }
   }
 }
@@ -204,16 +249,23 @@ __global__ void k_batch_reset(BatchHeader *hdr) {
   if (threadIdx.x == 0) {
     hdr->next = 0;
     hdr->next_oz = 0;
+    hdr->busy_oz = 0;
+    hdr->back = 0;
     hdr->bad = 0;
     hdr->first_bad = 0x7fffffff;
   }
 }
 
+// A launch of nothing: a grid that follows another at once is placed on the SMs
+// drained by then, two CTAs on some and none on others (200 problems, all of
+// the second pass: 2.3 ms against 1.96).
+__global__ void k_batch_drain() {}
+
 // Launch shape per device and precision, fixed on first use (before any
 // capture): grid = resident CTAs per SM x SMs.
 struct LaunchCfg {
   int grid = 0;                // of the pass every element type has
-  int grid_oz = 0;             // of the tensor-core pass
+  int grid_oz = 0;             // of the tensor-core pass (0: none)
   cudaError_t err = cudaSuccess;
 };
 static std::mutex g_cfg_mu;
@@ -259,9 +311,10 @@ static size_t work_bytes(int grid) {
   return sizeof(BatchHeader) + sizeof(R) * (size_t)grid * kScrElems;
 }
 
+// loops: every problem on the SIMT loops (the autotuner)
 template <typename R>
 static int batched_launch(int nprob, const void *probs, const int *order, R *A, R *B, void *work, size_t lwork,
-                          cudaStream_t st) {
+                          cudaStream_t st, bool loops = false) {
   if (nprob < 0) return -1;
   if (nprob > 0 && !probs) return -2;
   if (nprob > 0 && !order) return -3;
@@ -276,14 +329,25 @@ static int batched_launch(int nprob, const void *probs, const int *order, R *A, 
   k_batch_reset<<<1, 32, 0, st>>>(hdr);
   count_launch();
   if (nprob > 0) {
+    // no more problems than SMs: one CTA per SM is all there is to have
+    bool all = loops || !std::is_same<R, double>::value;
     if constexpr (std::is_same<R, double>::value) {
-      k_batched_gels<R, true><<<std::min(c.grid_oz, nprob), TQR_THREADS, kBatchDynSmem<true>, st>>>(
-          nprob, (const BatchProblem *)probs, order, A, B, hdr, scratch);
+      if (!loops) {
+        all = nprob <= c.grid_oz;
+        k_batched_gels<R, true><<<std::min(c.grid_oz, nprob), TQR_THREADS, kBatchDynSmem<true>, st>>>(
+            nprob, (const BatchProblem *)probs, order, A, B, hdr, scratch, all);
+        count_launch();
+      }
+    }
+    if (loops || !std::is_same<R, double>::value || !all) {
+      if (!all) {
+        k_batch_drain<<<1, 32, 0, st>>>();
+        count_launch();
+      }
+      k_batched_gels<R, false><<<std::min(c.grid, nprob), TQR_THREADS, kBatchDynSmem<false>, st>>>(
+          nprob, (const BatchProblem *)probs, order, A, B, hdr, scratch, all);
       count_launch();
     }
-    k_batched_gels<R, false><<<std::min(c.grid, nprob), TQR_THREADS, kBatchDynSmem<false>, st>>>(
-        nprob, (const BatchProblem *)probs, order, A, B, hdr, scratch);
-    count_launch();
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
@@ -367,7 +431,7 @@ static int residual_launch(int nprob, const void *probs, const R *A0, const R *B
 }
 
 // ---------------------------------------------------------------------------
-// Autotuner table: (ib, strip width) per column-count class
+// Autotuner table: (ib, strip width) of the SIMT loops per column-count class
 // n in (0,32], (32,64], (64,128], (128,256], (256,512].
 // ---------------------------------------------------------------------------
 constexpr int kClasses = 5;
@@ -407,7 +471,7 @@ static int autotune(cudaStream_t st, int force) {
   LaunchCfg c = launch_cfg<R>();
   if (c.err != cudaSuccess) return (int)c.err;
   // class representatives (m, n) and candidate (ib, nw)
-  const int shape[kClasses][2] = {{64, 24}, {160, 48}, {256, 96}, {384, 192}, {512, 384}};
+  const int shape[kClasses][2] = {{64, 24}, {112, 48}, {256, 96}, {384, 192}, {512, 384}};
   const Tune cand[6] = {{8, 8}, {16, 8}, {16, 16}, {32, 8}, {32, 16}, {24, 16}};
   const int kr = 4;
   const int np = 2 * c.grid;   // two waves of the persistent grid
@@ -446,7 +510,7 @@ static int autotune(cudaStream_t st, int force) {
         k_fill_uniform<R><<<1024, 256, 0, st>>>((long long)np * m * n, 1234 + rep, dA);
         k_fill_uniform<R><<<256, 256, 0, st>>>((long long)np * m * kr, 99 + rep, dB);
         chk(cudaEventRecord(e0, st));
-        if (rc == 0) rc = batched_launch<R>(np, dprobs, dorder, dA, dB, work, wb, st);
+        if (rc == 0) rc = batched_launch<R>(np, dprobs, dorder, dA, dB, work, wb, st, true);
         chk(cudaEventRecord(e1, st));
         chk(cudaEventSynchronize(e1));
         float ms = 0;
@@ -627,7 +691,7 @@ int tqr_batched_graph(int dtype_bytes, int nprob, const void *problems, const in
   if (rc == 0) {
     *graph_exec = (void *)ex;
     std::lock_guard<std::mutex> l(g_graph_mu);
-    g_graph_kernels[*graph_exec] = dtype_bytes == 8 ? 3 : 2;   // reset and the passes
+    g_graph_kernels[*graph_exec] = dtype_bytes == 8 && nprob > c.grid_oz ? 4 : 2;   // reset and the passes
   }
   return rc;
 }
