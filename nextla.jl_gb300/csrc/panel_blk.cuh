@@ -30,6 +30,8 @@
 // reflectors rounded to FP32 the line is 2^-30.  Elements whose fixed point
 // did not change keep their bits.
 #pragma once
+#include <new>
+
 #include "common.cuh"
 #include "oz_digits.cuh"
 
@@ -48,7 +50,8 @@ constexpr size_t kScale = kG8 + 64 * 8;                 // 32 ints
 constexpr size_t kWd = kScale + 32 * 4;                 // kD planes x 32 columns x 8 halves
 constexpr size_t kW1 = kWd + oz::kD * 512;              // 32 x 8 doubles
 constexpr size_t kWp = kW1 + 32 * 8 * 8;                // 8 x 384 int64 (then G, Y: 2 x 384 doubles)
-constexpr size_t kScratch = kWp + 8 * 384 * 8;
+constexpr size_t kOrig = kWp + 8 * 384 * 8;             // the caller's Orig, out of the registers' way
+constexpr size_t kScratch = kOrig + 64;
 
 // Panels the blocked loop takes; a property of the panel alone, so every
 // driver of the same factorisation takes the same path.
@@ -143,7 +146,7 @@ __device__ __forceinline__ void v_digits(const double *P, int ldp, int r0, int c
 template <int FORM, typename Orig>
 __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, int rs, double *Ts, int ldts, int m,
                                              int k, int nc, int tt, bool round32, bool zero_t_on_skip, double *tau,
-                                             unsigned char *scr, Orig orig) {
+                                             unsigned char *scr, const Orig &orig) {
   using namespace blk;
   constexpr int D = oz::kD;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -158,7 +161,9 @@ __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, i
   long long *const Wp = reinterpret_cast<long long *>(scr + kWp);
   unsigned long long *const X = reinterpret_cast<unsigned long long *>(P);
   const int nch = (m + 255) >> 8;                       // 256-row chunks
+  static_assert(sizeof(Orig) <= 64, "the caller's Orig in shared memory");
   if (k <= 0) return true;
+  if (tid == 0) new (scr + kOrig) Orig(orig);
 
   // ---- column scales: eight threads a column ----
   {
@@ -230,26 +235,21 @@ __device__ __noinline__ bool columns_blk_f64(double *P, int ldp, double *rowb, i
   for (int j0 = 0; j0 < nc; j0 += kW) {
     const int w = min(kW, nc - j0);
     double *const T8s = T8 + (j0 / kW) * 64;            // T8s[q + 8 p]
-    if (j0 > 0)
+    if (j0 > 0) {
+      // a rolled loop, and orig's address from shared memory: eight loads in
+      // flight here cost the strips of the same kernel their registers
+      // (8192^2 189.6 ms against 172.1)
+      const Orig &org = *reinterpret_cast<const Orig *>(scr + kOrig);
       for (int r = tid; r < m; r += TQR_THREADS) {
-        double *const p = P + (size_t)j0 * ldp + r;
-        double x[kW], o[kW];
-#pragma unroll
-        for (int c = 0; c < kW; ++c)
-          if (c < w) {
-            x[c] = p[(size_t)c * ldp];
-            o[c] = orig(r, j0 + c);
-          }
-#pragma unroll
-        for (int c = 0; c < kW; ++c)
-          if (c < w) {
-            const long long f = __double_as_longlong(x[c]) - (long long)oz::kBias;
-            x[c] = f == oz::to_fixed<true>(o[c], sc2[j0 + c]) ? o[c] : oz::from_fixed(f, sc2[j0 + c]);
-          }
-#pragma unroll
-        for (int c = 0; c < kW; ++c)
-          if (c < w) p[(size_t)c * ldp] = x[c];
+        double *p = P + (size_t)j0 * ldp + r;
+#pragma unroll 2
+        for (int c = 0; c < w; ++c, p += ldp) {
+          const double o = org(r, j0 + c);
+          const long long f = __double_as_longlong(*p) - (long long)oz::kBias;
+          *p = f == oz::to_fixed<true>(o, sc2[j0 + c]) ? o : oz::from_fixed(f, sc2[j0 + c]);
+        }
       }
+    }
     __syncwarp();                                       // a thread's rows are its warp's rows
 
     auto dots = [&](int i, int lo) {                    // part[warp][j] = sum over the warp's rows >= lo
