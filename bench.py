@@ -1488,8 +1488,12 @@ def main():
         except (OSError, ValueError, KeyError, TypeError):
             pass
     split_peak = half_peak / 28.0
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    mma_sync_split = 2.0 * 1024 * sms * 2.07e9 / 28.0 / 1e12      # 1024 multiply-adds a clock and SM, 2070 MHz
     roofline = {"bound": "fp16_tensor_exact_split", "achieved": achieved, "peak": split_peak, "unit": "TFLOP/s",
                 "frac": (achieved / split_peak) if achieved else None, "traffic": traffic,
+                "mma_sync_split_tflops": mma_sync_split,
+                "frac_of_mma_sync_split": (achieved / mma_sync_split) if achieved else None,
                 "fp64_simt_tflops": peak, "frac_of_fp64_simt": (achieved / peak) if achieved else None,
                 "fp64_mma_tflops": mma_peak,
                 "frac_of_fp64_mma": (achieved / mma_peak) if (achieved and mma_peak) else None,

@@ -620,7 +620,8 @@ int tqr_stile_geqrf_dag_f64p(int m, int n, int nb, int ib, float *A, int lda, fl
  * the strip width nw taken from the tuning table, and `order`, the problems by
  * decreasing flops; a_elems, b_elems are the packed lengths.  Returns
  * -(1000 + q) if problem q is out of range.
- * tqr_?batched_gels: one persistent launch (plus a counter reset) over the
+ * tqr_?batched_gels: one persistent launch (plus a counter reset; a double
+ * batch of more problems than SMs takes two) over the
  * device copies of the descriptors and order; work (256-byte aligned,
  * tqr_batched_worksize bytes) holds the counter and per-CTA scratch.
  * Descriptors the kernel finds out of range are skipped and counted:
@@ -628,8 +629,9 @@ int tqr_stile_geqrf_dag_f64p(int m, int n, int nb, int ib, float *A, int lda, fl
  * stream).  No allocation, no host synchronisation.
  * tqr_batched_graph: captures the same launch into an instantiated CUDA graph
  * (cudaGraphExec_t) for replay with tqr_batched_graph_launch.
- * tqr_batched_autotune: times every (ib, nw) candidate on synthetic problems
- * of each column-count class and stores the fastest in the table (allocates;
+ * tqr_batched_autotune: times every (ib, nw) candidate of the SIMT loops (double
+ * problems of 160 x 64 and more run on the tensor cores, in blocks of 32) on
+ * synthetic problems of each column-count class and stores the fastest in the table (allocates;
  * call it before planning and outside any capture); tqr_batched_tuning reads
  * the table entry for a column count.
  * tqr_?batched_residual: per problem ||A^T (B - A X)||_F /

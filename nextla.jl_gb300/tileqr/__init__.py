@@ -524,7 +524,7 @@ def tile_geqrf(A, nb=256, ib=32, T=None, tau=None, dag=True):
 
     dag=True runs the single persistent-kernel schedule when the shape allows
     it (scratch from a cached workspace; a matrix that is not whole tiles is
-    extended to whole ones), otherwise the stream driver; both give the same
+    extended to whole ones where that pays), otherwise the stream driver; both give the same
     bits on whole tiles."""
     import ctypes
     m, n = A.shape
